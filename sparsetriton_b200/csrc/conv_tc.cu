@@ -196,8 +196,6 @@ struct Params2 {
   uint32_t idesc;
   int out_kind;
   int idx_bytes;           // shared memory for staged map entries (0 with a tile plan)
-  int n_slots, slot_bytes; // planned_gather_kernel: ring of slots
-  int part;                // planned_gather_kernel: sub tiles per slot
   int w_flip;              // 1: offset k multiplies with W[K-1-k] (feature gradient of a submanifold layer over its own map)
   int dbg;                 // timing experiments only (wrong results): 1 no proxy fence, 2 no MMA, 4 no row copies, 8 no zero-fill copies
 };
@@ -281,7 +279,7 @@ __global__ void __launch_bounds__(kGatherThreads, 1) gather2_kernel(const Params
     auto producer_sync = [&]() {
       __syncwarp();
       if (lane == 0) mbar_arrive(smem_u32(&ctl->group_bar));
-      ok = mbar_wait_warp(smem_u32(&ctl->group_bar), group_phase, abort_flag, 28, lane) && ok;
+      ok = mbar_wait_all(smem_u32(&ctl->group_bar), group_phase, abort_flag, 28) && ok;
       group_phase ^= 1u;
     };
     long long t_pref = 0, t_acq_a = 0, t_acq_w = 0, t_total0 = PROF_CLOCK(), t_push = 0, t_copy = 0;
@@ -296,7 +294,7 @@ __global__ void __launch_bounds__(kGatherThreads, 1) gather2_kernel(const Params
       const long long c0 = PROF_CLOCK();
       queue.flush(lane);
       ++n_flush;
-      const bool r = mbar_wait_warp(bar, parity, abort_flag, where, lane);
+      const bool r = mbar_wait_all(bar, parity, abort_flag, where);
       if (where == 21) t_acq_w += PROF_CLOCK() - c0; else t_acq_a += PROF_CLOCK() - c0;
       return r;
     };
@@ -1162,20 +1160,19 @@ static bool fill_params2(tc::Params2* p, int dtype, const void* in, const void* 
     if (e && atoi(e) && sub >= 2 && 2 * sub * c_acc > 512) sub /= 2;
   }
 #endif
-  p->acc_bufs = (2 * sub * c_acc <= 512) ? 2 : 1;
   const int64_t n_tiles = (n_rows + tc::kTileM - 1) / tc::kTileM;
-  // small problems: do not leave SMs idle for the sake of sharing
-  while (sub > 1 && (n_tiles + sub - 1) / sub < sm_count()) --sub;
+  // Super tiles cost very different amounts of work (1 to K offsets): keep two and a half of them per SM or more, at the
+  // price of more copies of W.  (850 lidar tiles, 64 -> 32: S = 4 / 2 / 1 takes 37 / 37 / 33 us; 605 tiles, 64 -> 64: 44 / 39 /
+  // 33; 1563 tiles of 24 offsets each, 16 -> 32: 97 / 113 / 140; 6565 lidar tiles, 32 -> 32: 86 / 97 / 127.)
+  while (sub > 1 && 2 * n_tiles < 5 * (int64_t)sub * sm_count()) sub = sub > 2 ? 2 : 1;
   p->sub = sub;
+  p->acc_bufs = (2 * sub * c_acc <= 512) ? 2 : 1;
   p->n_super = (n_tiles + sub - 1) / sub;
   int cols = 32;
   while (cols < p->acc_bufs * sub * c_acc) cols <<= 1;
   p->tmem_cols = cols;
   p->w_slots = 3;
   p->idx_bytes = planned ? 0 : tc::kIdxTileBytes;
-  p->n_slots = 0;
-  p->slot_bytes = 0;
-  p->part = 1;
   p->w_flip = 0;
   const int budget = 222 * 1024 - p->idx_bytes;
   int a_stages = (budget - p->w_slots * p->w_slot_bytes) / tc::kABlockBytes;
@@ -1185,9 +1182,9 @@ static bool fill_params2(tc::Params2* p, int dtype, const void* in, const void* 
     a_stages = (budget - p->w_slots * p->w_slot_bytes) / tc::kABlockBytes;
     if (a_stages > tc::kMaxAStages) a_stages = tc::kMaxAStages;
   }
-  if (a_stages < (planned ? tc::kProducerWarps : 2)) return false;
-  // slot ownership by index needs whole rounds: of the four TMA-issuing warps or of the cp.async groups
-  a_stages -= a_stages % (planned ? tc::kProducerWarps : tc::kGatherGroups);
+  if (a_stages < (planned ? tc::kRowGroups + 1 : 2)) return false;
+  // gather2_kernel owns its stages by index: whole rounds of its producer groups
+  if (!planned) a_stages -= a_stages % tc::kGatherGroups;
   p->a_stages = a_stages;
   const uint32_t fmt = dtype == ST_F16 ? 0u : (dtype == ST_BF16 ? 1u : 2u);
   p->idesc = (1u << 4) | (fmt << 7) | (fmt << 10) | ((uint32_t)p->b_mn_major << 16) | ((uint32_t)(c_acc >> 3) << 17) |
@@ -1297,77 +1294,32 @@ static int launch_gather(tc::Params2 p, const Map& map, cudaStream_t stream) {
   return check_launch("tc gather");
 }
 
-// A stored map in tile-plan form: the TMA-fed kernel when the tensors can be described to the copy
-// engine (16-byte aligned bases and row pitches) and two whole-offset slots fit in shared memory,
-// else the cp.async producers of gather2_kernel over the same plan.
+// A stored map in tile-plan form.  A row warp announces a stage when its group's next one is under way, so the ring must be
+// longer than the number of groups.  planned_gather_kernel when the weights can be described to the copy engine and the
+// rows are whole 16-byte pieces, else gather2_kernel over the same plan.
 static int launch_planned(tc::Params2 p, const tc::PlannedRows& map, cudaStream_t stream) {
-  CUtensorMap in_desc, w_desc;
-  memset(&in_desc, 0, sizeof(in_desc));
+  CUtensorMap w_desc;
   memset(&w_desc, 0, sizeof(w_desc));
-  // Two CTAs per SM (experiment switch of instrumented builds): super tiles of at most two row tiles whose
-  // accumulators take at most half of TMEM, rings cut to half of the shared memory, twice the CTAs.  Measured
-  // slower on every layer tried (64 -> 128 k3 s2 forward 0.33 -> 0.47 ms, dgrad 0.25 -> 0.44 ms; submanifold
-  // 32..256 channels 1.5-1.8x slower): what bounds these kernels is the copy engine's rate of row gathers per SM,
-  // which two half-size pipelines share, while each W slice is then fetched for two row tiles instead of four.
-  int smem_budget = 222 * 1024;
-  int ctas_per_sm = 1;
-#ifdef ST_TC_PROFILE
-  {
-    const char* e = getenv("ST_TC_HALF");
-    if (e && atoi(e)) {
-      const int64_t n_tiles = (p.n_rows + tc::kTileM - 1) / tc::kTileM;
-      int sub = p.sub < 2 ? p.sub : 2;
-      while (sub > 1 && sub * p.c_acc > 256) --sub;
-      if (sub * p.c_acc <= 256) {
-        p.sub = sub;
-        p.n_super = (n_tiles + sub - 1) / sub;
-        p.acc_bufs = (2 * sub * p.c_acc <= 256) ? 2 : 1;
-        int cols = 32;
-        while (cols < p.acc_bufs * sub * p.c_acc) cols <<= 1;
-        p.tmem_cols = cols;
-        smem_budget = 110 * 1024;
-        ctas_per_sm = 2;
+  const bool planned = g_tma_enabled && p.a_stages > tc::kRowGroups && p.n_src > 0 && p.n_src < 0x7FFFFFFFll &&
+                       !(reinterpret_cast<uintptr_t>(p.in) & 15) && (p.c_red * p.esize) % 16 == 0 &&
+                       make_weight_desc(&w_desc, p.w, (int64_t)p.K * p.w_rows, p.w_cols, p.esize, p.out_kind,
+                                        p.b_mn_major ? 128 / p.esize : p.w_rows, p.b_mn_major && p.esize == 4);
+  if (!planned) return launch_gather(p, map, stream);
+  const size_t smem = (size_t)p.w_slots * p.w_slot_bytes + (size_t)p.a_stages * tc::kABlockBytes + sizeof(tc::Control3) + 1024;
+  auto kernel = p.esize == 2 ? tc::planned_gather_kernel<2> : tc::planned_gather_kernel<4>;
+  static bool configured[kMaxDevices] = {};
+  if (!configured[current_device()]) {
+    for (auto k : {tc::planned_gather_kernel<2>, tc::planned_gather_kernel<4>}) {
+      cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
+      if (e != cudaSuccess) {
+        set_error("tc planned gather: cannot raise the dynamic shared memory limit: %s", cudaGetErrorString(e));
+        return ST_ERR_CUDA;
       }
     }
+    configured[current_device()] = true;
   }
-#endif
-  p.part = p.sub;                        // smaller parts (more slots in flight) were measured slower
-#ifdef ST_TC_PROFILE
-  {
-    const char* e = getenv("ST_TC_PART");
-    if (e && atoi(e) >= 1 && atoi(e) <= p.sub) p.part = atoi(e);
-  }
-#endif
-  int n_slots = 0;
-  for (;;) {
-    p.slot_bytes = p.w_slot_bytes + p.part * tc::kABlockBytes;
-    n_slots = (int)((smem_budget - (int)sizeof(tc::Control3)) / p.slot_bytes);
-    if (n_slots > tc::kMaxSlots3) n_slots = tc::kMaxSlots3;
-    // the slot that carries an offset's W slice is held until the offset's last item: the ring must
-    // have room for all of an offset's items
-    if (n_slots >= (p.sub + p.part - 1) / p.part || p.part >= p.sub) break;
-    ++p.part;
-  }
-  p.n_slots = n_slots;
-  const bool tma = g_tma_enabled && n_slots >= 2 && p.n_src > 0 &&
-                   make_gather_desc(&in_desc, p.in, p.n_src, p.c_red, p.esize, p.out_kind) &&
-                   make_weight_desc(&w_desc, p.w, (int64_t)p.K * p.w_rows, p.w_cols, p.esize, p.out_kind,
-                                    p.b_mn_major ? 128 / p.esize : p.w_rows, p.b_mn_major && p.esize == 4);
-  if (!tma) return launch_gather(p, map, stream);
-  const size_t smem = (size_t)p.n_slots * p.slot_bytes + sizeof(tc::Control3) + 1024;
-  auto kernel = p.esize == 2 ? tc::planned_gather_kernel<2> : tc::planned_gather_kernel<4>;
-  static bool configured[2][kMaxDevices] = {};
-  if (!configured[p.esize == 4][current_device()]) {
-    cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
-    if (e != cudaSuccess) {
-      set_error("tc planned gather: cannot raise the dynamic shared memory limit: %s", cudaGetErrorString(e));
-      return ST_ERR_CUDA;
-    }
-    configured[p.esize == 4][current_device()] = true;
-  }
-  const int64_t max_ctas = (int64_t)ctas_per_sm * sm_count();
-  int64_t grid = p.n_super < max_ctas ? p.n_super : max_ctas;
-  kernel<<<(unsigned)grid, tc::kThreads, smem, stream>>>(p, map, in_desc, w_desc);
+  const int64_t grid = p.n_super < sm_count() ? p.n_super : sm_count();
+  kernel<<<(unsigned)grid, tc::kGather3Threads, smem, stream>>>(p, map, w_desc);
   note_launches(1);
   return check_launch("tc planned gather");
 }

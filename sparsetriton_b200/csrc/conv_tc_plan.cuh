@@ -1,63 +1,134 @@
-// Gather kernel for a stored map in tile-plan form, fed by TMA.  Included by conv_tc.cu (one
-// translation unit: the device status word and the PTX wrappers are file-local there).
+// Gather kernel for a stored map in tile-plan form.  Included by conv_tc.cu (one translation unit: the
+// device status word and the PTX wrappers are file-local there).
 //
 //   OUT[order[r], :] = sum_k  IN[tmap(r, k), :] . B_k
 //
-// Same roles as gather2_kernel (warps 0-3 epilogue, warp 4 MMA issuer, warps 5-8 producers) and the
-// same super tiles of S row tiles that share the copies of W, but the unit that travels through
-// shared memory is a whole kernel offset of the super tile:
+// Super tiles of S row tiles, whose accumulators sit side by side in TMEM, share the copies of W: for every offset k
+// (and 128-byte block kb of the reduction) that occurs in the super tile, W[k] travels once through a ring of W slots, and
+// each sub tile that has the offset sends one stage of 128 gathered rows through the ring of row stages.
 //
-//   slot = [ W slice of (k, kb) | rows of sub tile 0 | ... | rows of sub tile S-1 ]      one mbarrier
+// Warps 0-3 drain accumulators, warp 4 issues the MMAs, warp 5 fetches W slices by TMA, warps 6-21 fetch rows with
+// 16-byte cp.async: four groups of four warps take the stages in turn, a warp has 32 rows of a stage.  All of them walk
+// the tile masks themselves, so nothing but data and barriers goes through shared memory.
 //
-// or, to have more and smaller slots in flight, a part of it: the super tile's S sub tiles are dealt
-// in parts of P; the offset's first item carries the W slice and its slot is held back until the
-// offset's last item has been multiplied.
+// What bounds it: bringing rows into shared memory.  A loop that does nothing else (148 CTAs, random rows) takes, per
+// stage of 128 rows, with tile::gather4 612-743 cycles when every row exists and 1180 (128-byte rows) to 1880
+// (64-byte rows) when half of them are absent -- out-of-range rows are what the copy engine is slowest at -- and with
+// cp.async from 16 warps 265-344 (128-byte rows) and 160-207 (64-byte rows), absent or not, from tables of 8 to 160 MB.
+// Eight warps reach half of that: it is latency times warps, hence 16, and hence stages of one sub tile: slots of a whole
+// super tile's rows (two or three in the ring, mostly half used) left too little in flight.
 //
-// Producer warp w fetches the rows of sub tile w with 32 tile::gather4 copies (lane l: rows 4l..4l+3;
-// "-1" and rows past the end of the source are out of bounds and arrive as zeros); warp 0 also
-// fetches the W slice with one or two tiled copies; each warp announces its own bytes on the slot's
-// mbarrier.  The MMA
-// thread then waits once, issues up to 4 x S tcgen05.mma and commits once per offset.  With one wait
-// / commit per 16-KB row stage (gather2_kernel) the MMA thread's own instruction stream was the
-// bottleneck (about 600 cycles of bookkeeping for 256 cycles of tensor work).
-//
-// Every producer warp waits for every slot's release, whether or not its sub tile takes part in the
-// offset: an mbarrier wait names a phase only by its parity, so a warp that skipped laps of a slot
-// could be two laps ahead of the consumer and mistake an old phase for the one it needs.
+// Hand-over of a stage: 128 arrivals would serialise on its mbarrier, so a warp closes its share of a stage with
+// cp.async.commit_group and arrives for it (one lane) when its next share is on its way.  (Two shares on their way: up to
+// 6 % slower, a stage then waits for one eight stages behind it.)  The warp that issues the MMAs fences the proxies.
 #pragma once
 
 namespace st {
 namespace tc {
 
-constexpr int kMaxSlots3 = 6;
+constexpr int kRowGroups = 4, kRowGroupWarps = 4;             // warps that fetch rows
+constexpr int kWarpW = kMmaWarp + 1;                          // the warp that fetches W slices
+constexpr int kFirstRowWarp = kWarpW + 1;
+constexpr int kGather3Threads = (kFirstRowWarp + kRowGroups * kRowGroupWarps) * 32;
 
 struct __align__(8) Control3 {
-  unsigned long long full[kMaxSlots3], empty[kMaxSlots3];
+  unsigned long long a_full[kMaxAStages], a_empty[kMaxAStages];
+  unsigned long long w_full[kMaxWSlots], w_empty[kMaxWSlots];
   unsigned long long acc_full[2], acc_empty[2];
-  // bits 0-3 sub tiles that take part, bits 4-7 those whose accumulator starts here, bits 8-11 K-steps,
-  // bit 12 end of super tile (no data), bit 13 the slot carries the offset's W slice, bit 14 last item
-  // of the offset, bits 16-17 which part of the super tile the slot's rows belong to
-  uint32_t info[kMaxSlots3];
   uint32_t tmem_base;
   int abort_flag;
 };
 
+// The work of this CTA in order: item(tile0, k, kb, users, fresh) for every occupied (offset, 128-byte block) of a
+// super tile (users: the sub tiles that have the offset; fresh: those whose accumulator starts here), between
+// begin(tile0) and end(tile0).  Stops when one of them returns false.
+template <typename Begin, typename Item, typename End>
+__device__ __forceinline__ void walk_super_tiles(const Params2& p, const PlannedRows& map, int64_t n_tiles, Begin&& begin,
+                                                 Item&& item, End&& end) {
+  auto load_masks = [&](int64_t tile0, int word, uint32_t* m) {
+#pragma unroll
+    for (int s = 0; s < kMaxSub; ++s)
+      m[s] = (s < p.sub && tile0 + s < n_tiles) ? __ldg(map.tmask + (tile0 + s) * map.MW + word) : 0u;
+  };
+  // every lane loads the same words; the reduction tells the compiler so (uniform registers and branches)
+  auto uniform = [](uint32_t* m) {
+#pragma unroll
+    for (int s = 0; s < kMaxSub; ++s) m[s] = __reduce_or_sync(0xFFFFFFFFu, m[s]);
+  };
+  uint32_t next_m[kMaxSub];
+  load_masks((int64_t)blockIdx.x * p.sub, 0, next_m);
+  for (int64_t st_i = blockIdx.x; st_i < p.n_super; st_i += gridDim.x) {
+    const int64_t tile0 = st_i * p.sub;
+    uint32_t m[kMaxSub];
+#pragma unroll
+    for (int s = 0; s < kMaxSub; ++s) m[s] = next_m[s];
+    uniform(m);
+    if (st_i + gridDim.x < p.n_super) load_masks((st_i + gridDim.x) * p.sub, 0, next_m);
+    if (!begin(tile0)) return;
+    uint32_t touched = 0;
+    for (int word = 0; word < map.MW; ++word) {
+      if (word) {
+        load_masks(tile0, word, m);
+        uniform(m);
+      }
+      static_assert(kMaxSub == 4, "the masks of a super tile are combined by hand");
+      uint32_t m_any = m[0] | m[1] | m[2] | m[3];
+      while (m_any) {
+        const int j = __ffs(m_any) - 1;
+        m_any &= m_any - 1;
+        uint32_t users = 0;
+#pragma unroll
+        for (int s = 0; s < kMaxSub; ++s) users |= ((m[s] >> j) & 1u) << s;
+        for (int kb = 0; kb < p.k_blocks; ++kb)
+          if (!item(tile0, word * 32 + j, kb, users, kb == 0 ? (users & ~touched) : 0u)) return;
+        touched |= users;
+      }
+    }
+    if (!end(tile0)) return;
+  }
+}
+
+// A warp's 32 rows of a stage: 2^kLpr lanes share a row (16 bytes each).  All row numbers are exchanged before the first
+// copy: a shuffle behind a cp.async in the memory pipe waits for it (450 cycles per copy when they alternated).
+template <int kLpr>
+__device__ __forceinline__ void fetch_rows(uint32_t dst, int row0, int idx, const char* col, int pitch, int64_t n_src, int chunks,
+                                           int lane) {
+  constexpr int kRowsPer = 32 >> kLpr, kN = 1 << kLpr;
+  const int c = lane & (kN - 1), r_lane = lane >> kLpr;
+  int src[kN];
+#pragma unroll
+  for (int i = 0; i < kN; ++i) src[i] = __shfl_sync(0xFFFFFFFFu, idx, i * kRowsPer + r_lane);
+  col += c * 16;
+#pragma unroll
+  for (int i = 0; i < kN; ++i) {
+    const bool have = (uint32_t)src[i] < (uint32_t)n_src;                      // "-1" and rows past the source: zeros
+    const int row = row0 + i * kRowsPer + r_lane;
+    if (c < chunks)
+      cp_async16(dst + (uint32_t)row * 128u + ((uint32_t)swz16(c, row) << 4),
+                 col + (have ? (size_t)(uint32_t)src[i] * (uint32_t)pitch : 0), have ? 16u : 0u);
+  }
+}
+
 template <int ESIZE>
-__global__ void __launch_bounds__(kThreads, 1) planned_gather_kernel(const Params2 p, const PlannedRows map,
-                                                                     const __grid_constant__ CUtensorMap in_desc,
-                                                                     const __grid_constant__ CUtensorMap w_desc) {
+__global__ void __launch_bounds__(kGather3Threads, 1) planned_gather_kernel(const Params2 p, const PlannedRows map,
+                                                                            const __grid_constant__ CUtensorMap w_desc) {
   extern __shared__ unsigned char smem_raw[];
   const uint32_t raw = smem_u32(smem_raw);
   const uint32_t base = (raw + 1023u) & ~1023u;
   unsigned char* base_ptr = smem_raw + (base - raw);
-  Control3* ctl = reinterpret_cast<Control3*>(base_ptr + (size_t)p.n_slots * p.slot_bytes);
+  const uint32_t a_ring = base + (uint32_t)p.w_slots * (uint32_t)p.w_slot_bytes;
+  Control3* ctl = reinterpret_cast<Control3*>(base_ptr + (size_t)p.w_slots * p.w_slot_bytes + (size_t)p.a_stages * kABlockBytes);
   volatile int* abort_flag = &ctl->abort_flag;
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = __shfl_sync(0xFFFFFFFFu, (int)(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;
 
   if (threadIdx.x == 0) {
-    for (int s = 0; s < p.n_slots; ++s) {
-      mbar_init(smem_u32(&ctl->full[s]), kProducerWarps);
-      mbar_init(smem_u32(&ctl->empty[s]), 1);
+    for (int s = 0; s < p.a_stages; ++s) {
+      mbar_init(smem_u32(&ctl->a_full[s]), kRowGroupWarps);
+      mbar_init(smem_u32(&ctl->a_empty[s]), 1);
+    }
+    for (int s = 0; s < p.w_slots; ++s) {
+      mbar_init(smem_u32(&ctl->w_full[s]), 1);
+      mbar_init(smem_u32(&ctl->w_empty[s]), 1);
     }
     for (int b = 0; b < 2; ++b) {
       mbar_init(smem_u32(&ctl->acc_full[b]), 1);
@@ -77,221 +148,167 @@ __global__ void __launch_bounds__(kThreads, 1) planned_gather_kernel(const Param
   const int red_bytes = p.c_red * ESIZE;
   const int set_cols = p.sub * p.c_acc;                      // TMEM columns of one accumulator set
   const int64_t n_tiles = (p.n_rows + kTileM - 1) / kTileM;
+  auto nothing = [](int64_t) { return true; };
 
-  if (warp >= kFirstProducerWarp) {
-    // =============================================================== producers
-    const int pw = warp - kFirstProducerWarp;                // sub tile served by this warp
-    const int kr = 128 / ESIZE;
+  if (warp >= kFirstRowWarp) {
+    // =============================================================== rows
+    static_assert(kRowGroups == kMaxSub, "an offset has at most one stage per group");
+    const int group = (warp - kFirstRowWarp) / kRowGroupWarps;
+    const int row0 = (warp - kFirstRowWarp) % kRowGroupWarps * 32;
+    const char* in = static_cast<const char*>(p.in);
+    int sent = -1;                                            // stage whose copies are under way, not yet announced
+    int stage = 0, turn = 0;                                  // ring position and group of the next stage
+    uint32_t phase = 0;
+    bool ok = true;
+    int pend_stage = -1, pend_kb = 0, pend_idx = -1;
+    uint32_t pend_parity = 0;
+    auto run = [&]() {
+      ok = mbar_wait_all(smem_u32(&ctl->a_empty[pend_stage]), pend_parity ^ 1u, abort_flag, 31);
+      if (!ok) return;
+      const int chunks = min(128, red_bytes - pend_kb * 128) >> 4;             // 16-byte pieces of a row: 2, 4, 6 or 8
+      const uint32_t dst = a_ring + (uint32_t)pend_stage * kABlockBytes;
+      const char* col = in + pend_kb * 128;
+      if (chunks > 4) fetch_rows<3>(dst, row0, pend_idx, col, red_bytes, p.n_src, chunks, lane);
+      else if (chunks > 2) fetch_rows<2>(dst, row0, pend_idx, col, red_bytes, p.n_src, chunks, lane);
+      else fetch_rows<1>(dst, row0, pend_idx, col, red_bytes, p.n_src, chunks, lane);
+      cp_async_commit();
+      cp_async_wait_group<1>();                               // the share before this one has landed: announce it
+      __syncwarp();
+      if (sent >= 0 && lane == 0) mbar_arrive(smem_u32(&ctl->a_full[sent]));
+      sent = pend_stage;
+    };
+    walk_super_tiles(p, map, n_tiles, nothing, [&](int64_t tile0, int k, int kb, uint32_t users, uint32_t) {
+      const int n = __popc(users), mine = (group - turn) & (kRowGroups - 1);
+      if (mine < n) {
+        // this stage's row numbers are loaded now and its copies issued when the group's next stage comes up, so that
+        // the load overlaps the wait and copies of the one before
+        uint32_t u = users;
+        for (int i = 0; i < mine; ++i) u &= u - 1;
+        const int s = __ffs(u) - 1;
+        const int idx = __ldg(map.tmap + ((tile0 + s) * map.K + k) * (int64_t)kTileM + row0 + lane);
+        if (pend_stage >= 0) run();
+        const bool wrap = stage + mine >= p.a_stages;
+        pend_stage = wrap ? stage + mine - p.a_stages : stage + mine;
+        pend_parity = wrap ? phase ^ 1u : phase;
+        pend_kb = kb;
+        pend_idx = idx;
+      }
+      turn = (turn + n) & (kRowGroups - 1);
+      stage += n;
+      if (stage >= p.a_stages) {
+        stage -= p.a_stages;
+        phase ^= 1u;
+      }
+      return ok;
+    }, nothing);
+    if (pend_stage >= 0 && ok) run();
+    cp_async_wait_all();
+    __syncwarp();
+    if (sent >= 0 && lane == 0) mbar_arrive(smem_u32(&ctl->a_full[sent]));
+  } else if (warp == kWarpW) {
+    // =============================================================== W slices
     const int w_col_bytes = p.w_cols * ESIZE;
+    const int kr = 128 / ESIZE;
     const uint32_t w_bytes = p.b_mn_major ? (uint32_t)(((w_col_bytes + 127) >> 7) * kr * 128) : (uint32_t)(p.w_rows * 128);
     int slot = 0;
     uint32_t phase = 0;
-    bool ok = true;
-    struct Item {
-      int k, kb;
-      uint32_t users, fresh;   // sub tiles of this item (absolute bits)
-      int part;                // which group of p.part sub tiles
-      bool has_w, last;        // carries the W slice / is the offset's last item
-      int slot;
-      uint32_t parity;
-      bool marker, valid;
+    auto prefetch = [&](int64_t tile0) {
+      // the index lines of a super tile are one contiguous block of the plan: have the next one in L2
+      const int64_t next_tile0 = tile0 + (int64_t)gridDim.x * p.sub;
+      const int64_t lines = min(min((int64_t)p.sub, n_tiles - next_tile0) * map.K * 4, (int64_t)1024);   // of 128 bytes
+      const char* block = reinterpret_cast<const char*>(map.tmap + next_tile0 * map.K * (int64_t)kTileM);
+      for (int64_t l = lane; l < lines; l += 32) prefetch_l2(block + l * 128);
+      return true;
     };
-    Item pend{0, 0, 0u, 0u, 0, false, false, 0, 0u, false, false};
-    int4 pend_idx = make_int4(-1, -1, -1, -1);
-
-    auto run = [&](const Item& d, const int4& idx) {
-      ok = mbar_wait_warp(smem_u32(&ctl->empty[d.slot]), d.parity ^ 1u, abort_flag, 31, lane);
-      if (!ok) return;
-      const uint32_t bar = smem_u32(&ctl->full[d.slot]);
-      const uint32_t slot_base = base + (uint32_t)d.slot * (uint32_t)p.slot_bytes;
-      const bool copy_rows = !d.marker && !ST_DBG(p, 4) && ((d.users >> pw) & 1u);
+    walk_super_tiles(p, map, n_tiles, prefetch, [&](int64_t, int k, int kb, uint32_t, uint32_t) {
+      if (!mbar_wait_all(smem_u32(&ctl->w_empty[slot]), phase ^ 1u, abort_flag, 35)) return false;
       if (lane == 0) {
-        // Every producer warp arrives on every slot, announcing the bytes of its own copies first (a
-        // copy that completed before its bytes were announced would drive the count negative).
-        const bool copy_w = pw == 0 && d.has_w && !d.marker && !ST_DBG(p, 16);
-        if (pw == 0) {
-          const int valid_bytes = d.marker ? 0 : min(128, red_bytes - d.kb * 128);
-          ctl->info[d.slot] = d.users | (d.fresh << 4) | ((uint32_t)(valid_bytes >> 5) << 8) | (d.marker ? 0x1000u : 0u) |
-                              (d.has_w ? 0x2000u : 0u) | (d.last ? 0x4000u : 0u) | ((uint32_t)d.part << 16);
-        }
-        const uint32_t bytes = (copy_w ? w_bytes : 0u) + (copy_rows ? (uint32_t)kABlockBytes : 0u);
-        if (bytes) mbar_arrive_expect_tx(bar, bytes); else mbar_arrive(bar);
-        if (copy_w) {
-          const int kw = p.w_flip ? p.K - 1 - d.k : d.k;     // which W slice this offset multiplies with
-          if (p.b_mn_major) {
-            const int n_cb = (w_col_bytes + 127) >> 7;
-            for (int cb = 0; cb < n_cb; ++cb)
-              tma_load_2d(slot_base + (uint32_t)(cb * kr * 128), &w_desc, bar, cb * kr, kw * p.w_rows + d.kb * kr);
-          } else {
-            tma_load_2d(slot_base, &w_desc, bar, d.kb * kr, kw * p.w_rows);
-          }
+        const uint32_t bar = smem_u32(&ctl->w_full[slot]);
+        const uint32_t dst = base + (uint32_t)slot * (uint32_t)p.w_slot_bytes;
+        mbar_arrive_expect_tx(bar, w_bytes);
+        const int kw = p.w_flip ? p.K - 1 - k : k;             // which W slice this offset multiplies with
+        if (p.b_mn_major) {
+          const int n_cb = (w_col_bytes + 127) >> 7;
+          for (int cb = 0; cb < n_cb; ++cb)
+            tma_load_2d(dst + (uint32_t)(cb * kr * 128), &w_desc, bar, cb * kr, kw * p.w_rows + kb * kr);
+        } else {
+          tma_load_2d(dst, &w_desc, bar, kb * kr, kw * p.w_rows);
         }
       }
       __syncwarp();
-      if (copy_rows)
-        tma_gather4(slot_base + (uint32_t)p.w_slot_bytes + (uint32_t)(pw - d.part * p.part) * kABlockBytes +
-                        (uint32_t)lane * 512u,
-                    &in_desc, bar, d.kb * kr, idx.x, idx.y, idx.z, idx.w);
-    };
-    // Queue one item: its indices are loaded now and it is issued when the next one is queued, so the
-    // load overlaps the previous item's wait and copies.
-    auto emit_item = [&](int64_t tile0, const Item& d, bool zeros) {
-      int4 idx = make_int4(-1, -1, -1, -1);
-      if (!d.marker && !zeros && ((d.users >> pw) & 1u))
-        idx = __ldg(reinterpret_cast<const int4*>(map.tmap + ((tile0 + pw) * map.K + d.k) * (int64_t)kTileM) + lane);
-      if (pend.valid && ok) run(pend, pend_idx);
-      pend = d;
-      pend.slot = slot;
-      pend.parity = phase;
-      pend.valid = true;
-      pend_idx = idx;
-      if (++slot == p.n_slots) {
+      if (++slot == p.w_slots) {
         slot = 0;
         phase ^= 1u;
       }
-    };
-    // One offset of the super tile: an item per part (p.part sub tiles) that has a user; the first one
-    // carries the W slice, which the later ones read from its slot.
-    auto emit = [&](int64_t tile0, int k, int kb, uint32_t users, uint32_t fresh, bool marker, bool zeros) {
-      if (marker) {
-        emit_item(tile0, Item{0, 0, 0u, 0u, 0, false, false, 0, 0u, true, true}, false);
-        return;
-      }
-      const uint32_t part_bits = (1u << p.part) - 1u;
-      bool first = true;
-      for (int q = 0; q * p.part < p.sub; ++q) {
-        const uint32_t u = users & (part_bits << (q * p.part));
-        if (!u) continue;
-        const bool last = (users >> ((q + 1) * p.part)) == 0u;
-        emit_item(tile0, Item{k, kb, u, fresh & u, q, first, last, 0, 0u, false, true}, zeros);
-        first = false;
-      }
-    };
-    auto load_masks = [&](int64_t tile0, int word, uint32_t* m) {
-#pragma unroll
-      for (int s = 0; s < kMaxSub; ++s)
-        m[s] = (s < p.sub && tile0 + s < n_tiles) ? __ldg(map.tmask + (tile0 + s) * map.MW + word) : 0u;
-    };
-    uint32_t next_m[kMaxSub];
-    load_masks((int64_t)blockIdx.x * p.sub, 0, next_m);
-    for (int64_t st_i = blockIdx.x; st_i < p.n_super && ok; st_i += gridDim.x) {
-      const int64_t tile0 = st_i * p.sub;
-      uint32_t m0[kMaxSub];
-#pragma unroll
-      for (int s = 0; s < kMaxSub; ++s) m0[s] = next_m[s];
-      if (st_i + gridDim.x < p.n_super) {
-        const int64_t next_tile0 = (st_i + gridDim.x) * p.sub;
-        load_masks(next_tile0, 0, next_m);
-        // the index lines of a super tile are one contiguous block of the plan: have the next one in L2
-        const int64_t tiles = min((int64_t)p.sub, n_tiles - next_tile0);
-        const char* block = reinterpret_cast<const char*>(map.tmap + next_tile0 * map.K * (int64_t)kTileM);
-        const int64_t lines = min(tiles * map.K * 4, (int64_t)1024);               // 128-byte lines
-        for (int64_t l = (warp - kFirstProducerWarp) * 32 + lane; l < lines; l += kProducerThreads)
-          prefetch_l2(block + l * 128);
-      }
-      uint32_t touched = 0;
-      for (int word = 0; word < map.MW && ok; ++word) {
-        uint32_t m[kMaxSub], m_any = 0;
-        if (word == 0) {
-#pragma unroll
-          for (int s = 0; s < kMaxSub; ++s) m[s] = m0[s];
-        } else {
-          load_masks(tile0, word, m);
-        }
-#pragma unroll
-        for (int s = 0; s < kMaxSub; ++s) m_any |= m[s];
-        while (m_any && ok) {
-          const int j = __ffs(m_any) - 1;
-          m_any &= m_any - 1;
-          uint32_t users = 0;
-#pragma unroll
-          for (int s = 0; s < kMaxSub; ++s) users |= ((m[s] >> j) & 1u) << s;
-          for (int kb = 0; kb < p.k_blocks && ok; ++kb)
-            emit(tile0, word * 32 + j, kb, users, kb == 0 ? (users & ~touched) : 0u, false, false);
-          touched |= users;
-        }
-      }
-      // sub tiles that exist but never got a neighbour still have to write zeros
-      uint32_t untouched = 0;
-      for (int s = 0; s < p.sub; ++s)
-        if (tile0 + s < n_tiles && !((touched >> s) & 1u)) untouched |= 1u << s;
-      if (untouched && ok) emit(tile0, 0, 0, untouched, untouched, false, true);
-      if (ok) emit(tile0, 0, 0, 0u, 0u, true, false);                            // end of super tile
-    }
-    if (pend.valid && ok) run(pend, pend_idx);
+      return true;
+    }, nothing);
   } else if (warp == kMmaWarp) {
     // =============================================================== MMA issuer
-    if (lane == 0) {
-      int slot = 0;
-      uint32_t phase = 0;
+    // The whole warp runs this, converged, so that descriptors, ring positions and branches live in uniform registers, and
+    // one elected lane issues.  As a branch of one lane the same code took 950 cycles per stage (130 per MMA, moving
+    // its operands from vector to uniform registers), more than the copies or the MMAs themselves.
+    {
+      int stage = 0, slot = 0;
+      uint32_t phase = 0, w_phase = 0;
       uint32_t acc_phase[2] = {0, 0};
       int buf = 0;
-      bool ok = true;
       const uint32_t b_kstep16 = (p.b_mn_major ? (32 / ESIZE) * 128 : 32) >> 4;   // K-step advance, 16-byte units
       const uint32_t b_lbo = p.b_mn_major ? (uint32_t)(128 / ESIZE) * 128u : 16u;
       const bool b_base32 = p.b_mn_major && ESIZE == 4;
       const uint64_t a_desc_hi = smem_desc(0u, 16u, 1024u, 2u);
       const uint64_t b_desc_hi = smem_desc(0u, b_lbo, b_base32 ? 512u : 1024u, b_base32 ? 1u : 2u);
       const uint32_t idesc = p.idesc;
-      uint32_t w_lo = 0;
-      int held = -1;                                          // slot kept for its W slice
-      for (int64_t st_i = blockIdx.x; st_i < p.n_super && ok; st_i += gridDim.x) {
-        ok = mbar_wait(smem_u32(&ctl->acc_empty[buf]), acc_phase[buf] ^ 1u, abort_flag, 32);
-        if (!ok) break;
-        tc_fence_after();
-        for (;;) {
-          ok = mbar_wait(smem_u32(&ctl->full[slot]), phase, abort_flag, 33);
-          if (!ok) break;
-          const uint32_t info = ctl->info[slot];
+      walk_super_tiles(p, map, n_tiles,
+        [&](int64_t) {
+          const bool ok = mbar_wait_all(smem_u32(&ctl->acc_empty[buf]), acc_phase[buf] ^ 1u, abort_flag, 32);
           tc_fence_after();
-          const uint32_t slot_base = base + (uint32_t)slot * (uint32_t)p.slot_bytes;
-          if (info & 0x2000u) {                                  // the offset's W slice lives in this slot
-            w_lo = slot_base >> 4;
-            held = slot;
-          }
-          if (!(info & 0x1000u) && !ST_DBG(p, 2)) {
-            const int ksteps = (int)((info >> 8) & 15u);
-            const int part0 = (int)((info >> 16) & 3u) * p.part;
+          return ok;
+        },
+        [&](int64_t, int, int kb, uint32_t users, uint32_t fresh) {
+          if (!mbar_wait_all(smem_u32(&ctl->w_full[slot]), w_phase, abort_flag, 33)) return false;
+          const uint32_t w_lo = (base + (uint32_t)slot * (uint32_t)p.w_slot_bytes) >> 4;
+          const int ksteps = min(128, red_bytes - kb * 128) >> 5;
 #pragma unroll
-            for (int s = 0; s < kMaxSub; ++s) {
-              if (!((info >> s) & 1u)) continue;
-              const uint32_t a_lo = (slot_base + (uint32_t)p.w_slot_bytes + (uint32_t)(s - part0) * kABlockBytes) >> 4;
-              const uint32_t d_addr = tmem_base + (uint32_t)(buf * set_cols + s * p.c_acc);
-              const uint32_t fresh = ((info >> (4 + s)) & 1u) ? 0u : 1u;        // 0: the first MMA overwrites
+          for (int s = 0; s < kMaxSub; ++s) {
+            if (!((users >> s) & 1u)) continue;
+            if (!mbar_wait_all(smem_u32(&ctl->a_full[stage]), phase, abort_flag, 34)) return false;
+            fence_proxy_async();                                                 // rows were written by cp.async
+            tc_fence_after();
+            const uint32_t a_lo = (a_ring + (uint32_t)stage * kABlockBytes) >> 4;
+            const uint32_t d_addr = tmem_base + (uint32_t)(buf * set_cols + s * p.c_acc);
+            const uint32_t add = ((fresh >> s) & 1u) ? 0u : 1u;                  // 0: the first MMA overwrites
+            if (elect_one()) {
 #pragma unroll
               for (int ks = 0; ks < 4; ++ks) {
                 if (ks < ksteps) {
                   const uint64_t da = a_desc_hi | (uint64_t)(a_lo + ks * 2);
                   const uint64_t db = b_desc_hi | (uint64_t)(w_lo + ks * b_kstep16);
                   if (ESIZE == 2)
-                    mma_f16(d_addr, da, db, idesc, ks == 0 ? fresh : 1u);
+                    mma_f16(d_addr, da, db, idesc, ks == 0 ? add : 1u);
                   else
-                    mma_tf32(d_addr, da, db, idesc, ks == 0 ? fresh : 1u);
+                    mma_tf32(d_addr, da, db, idesc, ks == 0 ? add : 1u);
                 }
               }
+              mma_commit(smem_u32(&ctl->a_empty[stage]));
+            }
+            if (++stage == p.a_stages) {
+              stage = 0;
+              phase ^= 1u;
             }
           }
-          // A slot that holds the W slice stays with the consumer until the offset's last item is done.
-          if (info & 0x1000u) {
-            mma_commit(smem_u32(&ctl->empty[slot]));
-          } else if (info & 0x4000u) {
-            if (held >= 0 && held != slot) mma_commit(smem_u32(&ctl->empty[held]));
-            mma_commit(smem_u32(&ctl->empty[slot]));
-            held = -1;
-          } else if (held != slot) {
-            mma_commit(smem_u32(&ctl->empty[slot]));
-          }
-          if (++slot == p.n_slots) {
+          if (elect_one()) mma_commit(smem_u32(&ctl->w_empty[slot]));
+          if (++slot == p.w_slots) {
             slot = 0;
-            phase ^= 1u;
+            w_phase ^= 1u;
           }
-          if (info & 0x1000u) break;
-        }
-        if (!ok) break;
-        mma_commit(smem_u32(&ctl->acc_full[buf]));
-        acc_phase[buf] ^= 1u;
-        if (p.acc_bufs == 2) buf ^= 1;
-      }
+          return true;
+        },
+        [&](int64_t) {
+          if (elect_one()) mma_commit(smem_u32(&ctl->acc_full[buf]));
+          acc_phase[buf] ^= 1u;
+          if (p.acc_bufs == 2) buf ^= 1;
+          return true;
+        });
     }
     __syncwarp();
   } else {
@@ -300,6 +317,10 @@ __global__ void __launch_bounds__(kThreads, 1) planned_gather_kernel(const Param
     int buf = 0;
     bool ok = true;
     const int out_es = p.out_kind == ST_F32 ? 4 : 2;
+    auto zero = [](uint32_t (&v)[32]) {
+#pragma unroll
+      for (int i = 0; i < 32; ++i) v[i] = 0u;
+    };
     for (int64_t st_i = blockIdx.x; st_i < p.n_super && ok; st_i += gridDim.x) {
       // where this lane's rows go: known before the accumulators are ready, so fetched before the wait
       int64_t dst_rows[kMaxSub];
@@ -308,7 +329,13 @@ __global__ void __launch_bounds__(kThreads, 1) planned_gather_kernel(const Param
         const int64_t row = (st_i * p.sub + s) * (int64_t)kTileM + warp * 32 + lane;
         dst_rows[s] = (s < p.sub && p.order && row < p.n_rows) ? (int64_t)__ldg(p.order + row) : row;
       }
-      ok = mbar_wait(smem_u32(&ctl->acc_full[buf]), acc_phase[buf], abort_flag, 34, 256);
+      // sub tiles without any neighbour have no accumulator: their rows are zeros
+      uint32_t touched = 0;
+#pragma unroll
+      for (int s = 0; s < kMaxSub; ++s)
+        for (int word = 0; word < map.MW; ++word)
+          if (s < p.sub && st_i * p.sub + s < n_tiles && __ldg(map.tmask + (st_i * p.sub + s) * map.MW + word)) touched |= 1u << s;
+      ok = mbar_wait(smem_u32(&ctl->acc_full[buf]), acc_phase[buf], abort_flag, 40, 256);
       ok = __all_sync(0xFFFFFFFFu, ok);
       if (!ok) break;
       tc_fence_after();
@@ -319,15 +346,17 @@ __global__ void __launch_bounds__(kThreads, 1) planned_gather_kernel(const Param
         if ((st_i * p.sub + s) * (int64_t)kTileM >= p.n_rows) break;         // whole sub tile past the end
         char* out_row = static_cast<char*>(p.out) + (size_t)dst_rows[s] * p.c_acc * out_es;
         const uint32_t t_row = tmem_base + ((uint32_t)(warp * 32) << 16) + (uint32_t)(buf * set_cols + s * p.c_acc);
-        for (int c0 = 0; c0 < p.c_acc && !ST_DBG(p, 128); c0 += 32) {
+        for (int c0 = 0; c0 < p.c_acc; c0 += 32) {
           uint32_t v[32];
           if (p.c_acc - c0 >= 32) {
             tmem_ld32(t_row + c0, v);
             tmem_ld_wait();
-            if (row < p.n_rows && !ST_DBG(p, 64)) store_cols<32>(out_row, c0, p.out_kind, v);
+            if (!((touched >> s) & 1u)) zero(v);
+            if (row < p.n_rows) store_cols<32>(out_row, c0, p.out_kind, v);
           } else {
             tmem_ld16(t_row + c0, v);
             tmem_ld_wait();
+            if (!((touched >> s) & 1u)) zero(v);
             if (row < p.n_rows) store_cols<16>(out_row, c0, p.out_kind, v);
           }
         }
@@ -470,7 +499,7 @@ __global__ void __launch_bounds__(kThreads, 1) planned_wgrad_kernel(const WgradP
         if (!m) continue;
         // ---- the dY tile: rows order[tile * 128 + r], or one dense box when the rows lie in tile order
         if (p.dense_tiles) {
-          ok = mbar_wait_warp(smem_u32(&ctl->a_empty[a_slot]), a_phase ^ 1u, abort_flag, 35, lane);
+          ok = mbar_wait_all(smem_u32(&ctl->a_empty[a_slot]), a_phase ^ 1u, abort_flag, 35);
           if (!ok) break;
           const uint32_t bar = smem_u32(&ctl->a_full[a_slot]);
           const uint32_t slot_base = a_ring + (uint32_t)a_slot * (uint32_t)p.a_slot_bytes;
@@ -503,7 +532,7 @@ __global__ void __launch_bounds__(kThreads, 1) planned_wgrad_kernel(const WgradP
           if (pos + 1 >= p.n_rows) rows.y = -1;
           if (pos + 2 >= p.n_rows) rows.z = -1;
           if (pos + 3 >= p.n_rows) rows.w = -1;
-          ok = mbar_wait_warp(smem_u32(&ctl->a_empty[a_slot]), a_phase ^ 1u, abort_flag, 35, lane);
+          ok = mbar_wait_all(smem_u32(&ctl->a_empty[a_slot]), a_phase ^ 1u, abort_flag, 35);
           if (!ok) break;
           const uint32_t bar = smem_u32(&ctl->a_full[a_slot]);
           const uint32_t slot_base = a_ring + (uint32_t)a_slot * (uint32_t)p.a_slot_bytes;
@@ -533,7 +562,7 @@ __global__ void __launch_bounds__(kThreads, 1) planned_wgrad_kernel(const WgradP
           int4 idx = make_int4(-1, -1, -1, -1);
           if (my_j >= 0)
             idx = __ldg(reinterpret_cast<const int4*>(map.tmap + (tile * map.K + k_first + my_j) * (int64_t)kTileM) + lane);
-          ok = mbar_wait_warp(smem_u32(&ctl->b_empty[b_slot]), b_phase ^ 1u, abort_flag, 36, lane);
+          ok = mbar_wait_all(smem_u32(&ctl->b_empty[b_slot]), b_phase ^ 1u, abort_flag, 36);
           if (!ok) break;
           const uint32_t bar = smem_u32(&ctl->b_full[b_slot]);
           const uint32_t stage = b_ring + (uint32_t)b_slot * quad_bytes + (uint32_t)pw * (uint32_t)p.b_slot_bytes;
@@ -647,7 +676,7 @@ __global__ void __launch_bounds__(kThreads, 1) planned_wgrad_kernel(const WgradP
     bool ok = true;
     auto issue = [&](const Task& t, const int4& rows) {
       if (t.kind == 1) {
-        ok = mbar_wait_warp(smem_u32(&ctl->a_empty[t.slot]), t.parity ^ 1u, abort_flag, 35, lane);
+        ok = mbar_wait_all(smem_u32(&ctl->a_empty[t.slot]), t.parity ^ 1u, abort_flag, 35);
         if (!ok) return;
         const uint32_t bar = smem_u32(&ctl->a_full[t.slot]);
         const uint32_t slot_base = a_ring + (uint32_t)t.slot * (uint32_t)p.a_slot_bytes;
@@ -664,7 +693,7 @@ __global__ void __launch_bounds__(kThreads, 1) planned_wgrad_kernel(const WgradP
             tma_gather4(slot_base + (uint32_t)b * kABlockBytes + (uint32_t)lane * 512u, tile_desc, bar, tile_col0 + b * per_line,
                         rows.x, rows.y, rows.z, rows.w);
       } else {
-        ok = mbar_wait_warp(smem_u32(&ctl->b_empty[t.slot]), t.parity ^ 1u, abort_flag, 36, lane);
+        ok = mbar_wait_all(smem_u32(&ctl->b_empty[t.slot]), t.parity ^ 1u, abort_flag, 36);
         if (!ok) return;
         const uint32_t bar = smem_u32(&ctl->b_full[t.slot]);
         const uint32_t stage = b_ring + (uint32_t)t.slot * quad_bytes + (uint32_t)(p.quad == 1 ? 0 : pw) * (uint32_t)p.b_slot_bytes;

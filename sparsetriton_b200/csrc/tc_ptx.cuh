@@ -10,6 +10,7 @@
 namespace st {
 namespace tc {
 
+constexpr uint32_t kWaitHintNs = 1000000;                      // how long the hardware may suspend a waiting thread per poll
 constexpr long long kWaitCycles = 4000000000ll;                // ~2 s at 2 GHz
 
 // Sticky device-side status: [0] ST_DEV_* flags, [1] id of the wait that expired, [2] block, [3] spare.
@@ -28,10 +29,10 @@ __device__ __forceinline__ bool mbar_try(uint32_t bar, uint32_t parity) {
   uint32_t ok;
   asm volatile(
       "{\n\t.reg .pred p;\n\t"
-      "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+      "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, %3;\n\t"
       "selp.u32 %0, 1, 0, p;\n\t}"
       : "=r"(ok)
-      : "r"(bar), "r"(parity)
+      : "r"(bar), "r"(parity), "r"(kWaitHintNs)
       : "memory");
   return ok != 0;
 }
@@ -122,6 +123,32 @@ __device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t (&v)[32]) {
       : "memory");
 }
 __device__ __forceinline__ void tmem_ld_wait() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
+// One lane of the (converged) warp.
+__device__ __forceinline__ bool elect_one() {
+  uint32_t pred;
+  asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xFFFFFFFF;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(pred));
+  return pred != 0;
+}
+// Bounded wait of a whole warp: every lane polls, so that the warp stays converged.  (With one lane polling and the answer
+// broadcast, a warp that had to wait went on in fragments: the code behind the wait ran four to five times slower.)
+__device__ __forceinline__ bool mbar_wait_all(uint32_t bar, uint32_t parity, volatile int* abort_flag, int where) {
+  if (__all_sync(0xFFFFFFFFu, mbar_try(bar, parity))) return true;
+  const long long t0 = clock64();
+  for (;;) {
+    if (__all_sync(0xFFFFFFFFu, mbar_try(bar, parity))) return true;
+    if (__any_sync(0xFFFFFFFFu, *abort_flag != 0)) return false;
+    if (__any_sync(0xFFFFFFFFu, clock64() - t0 > kWaitCycles)) {
+      if (elect_one()) {
+        *abort_flag = 1;
+        if (atomicOr(&g_status[0], ST_DEV_TIMEOUT) == 0) {
+          g_status[1] = where;
+          g_status[2] = blockIdx.x;
+        }
+      }
+      return false;
+    }
+  }
+}
 // ---- TMA (bulk tensor copies).  The descriptor lives in kernel parameter space (__grid_constant__).
 __device__ __forceinline__ void mbar_arrive_expect_tx(uint32_t bar, uint32_t bytes) {
   asm volatile("{\n\t.reg .b64 t;\n\tmbarrier.arrive.expect_tx.shared::cta.b64 t, [%0], %1;\n\t}" ::"r"(bar), "r"(bytes)
@@ -187,14 +214,6 @@ struct StageQueue {
     clear();
   }
 };
-
-// Whole-warp bounded wait: lane 0 polls, the result is broadcast.
-__device__ __forceinline__ bool mbar_wait_warp(uint32_t bar, uint32_t parity, volatile int* abort_flag, int where,
-                                               int lane) {
-  int ok = 1;
-  if (lane == 0) ok = mbar_wait(bar, parity, abort_flag, where) ? 1 : 0;
-  return __shfl_sync(0xFFFFFFFFu, ok, 0) != 0;
-}
 
 // Named barrier 1 among the `Threads` producer threads.
 template <int Threads>
