@@ -81,8 +81,8 @@ int st_set_tensor_cores(int enable);
  * the same plan.  Results are identical. */
 int st_set_tma(int enable);
 
-/* 1 (default): the planned weight gradient copies dY into tile order once and loads its tiles as dense boxes; 0: it
- * gathers the rows of every tile through the row order (the earlier form, kept for comparison).  No reference counterpart. */
+/* Accepted and without effect: the planned weight gradient reads the rows of its dY tiles through the row order.  No
+ * reference counterpart. */
 int st_set_dense_tiles(int enable);
 
 /* ---------------------------------------------------------------- hash table ------------- */
@@ -245,11 +245,10 @@ int st_conv_wgrad_planned(int dtype, const void* X, const void* dY, const int32_
                           const int32_t* tmap, const uint32_t* tmask, void* dW, int64_t n_in, int64_t n_out, int K,
                           int cin, int cout, void* workspace, int64_t workspace_bytes, void* stream);
 
-/* st_conv_wgrad_planned in two calls, for a caller that runs the first on another stream beside the feature gradient.
- * On tensor-core shapes st_conv_wgrad_planned first copies dY into the plan's row order (scratch in its workspace), so
- * that the product loads each dY tile as one dense box; the copy depends on dY and row_order alone.
+/* st_conv_wgrad_planned over a copy of dY in the plan's row order, made by a call of its own (on another stream, say).
+ * st_conv_wgrad_planned itself makes no copy and is as fast.
  *   st_conv_wgrad_presort            makes that copy in `workspace`.  ST_ERR_UNSUPPORTED (nothing launched, no error
- *                                    text) when st_conv_wgrad_planned would make none for this layer: call
+ *                                    text) for a layer whose dY tiles are read once or twice: call
  *                                    st_conv_wgrad_planned as usual then.
  *   st_conv_wgrad_planned_presorted  the rest, with the same arguments and the same workspace, once the copy is
  *                                    complete on `stream` (an event of the caller's).  Same dW, bit for bit, as

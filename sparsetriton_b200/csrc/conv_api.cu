@@ -42,9 +42,10 @@ static int64_t wgrad_partial_bytes(int64_t n_out, int K, int cin, int cout) {
 }
 
 // Partials of whichever weight-gradient kernel would run, so one workspace serves both.
-// The tensor-core form also keeps a copy of dY in tile order behind its partials (see tc_conv_wgrad).
+// Behind the tensor-core form's partials there is room for a copy of dY in tile order (st_conv_wgrad_presort).
 static int64_t wgrad_sorted_offset(int dtype, int64_t n_out, int K, int cin, int cout) {
-  return align_up(tc_wgrad_partial_bytes(dtype, n_out, K, cin, cout), 256);
+  const int64_t plain = tc_wgrad_partial_bytes(dtype, n_out, K, cin, cout), planned = tc_wgrad_planned_bytes(dtype, n_out, K, cin, cout);
+  return align_up(plain > planned ? plain : planned, 256);
 }
 static int64_t wgrad_workspace_bytes(int dtype, int64_t n_out, int K, int cin, int cout) {
   int64_t simt = wgrad_partial_bytes(n_out, K, cin, cout);
@@ -128,7 +129,7 @@ int st_set_tma(int enable) {
 }
 
 int st_set_dense_tiles(int enable) {
-  tc_set_dense_tiles(enable != 0);
+  (void)enable;
   return ST_OK;
 }
 
@@ -264,10 +265,10 @@ static int wgrad_planned(int dtype, const void* X, const void* dY, const int32_t
   cudaStream_t s = (cudaStream_t)stream;
   if (n_out > 0 && tc_wgrad_supported(dtype, n_out, K, cin, cout)) {
     int chunks = 0;
-    void* sorted_rows = static_cast<char*>(workspace) + wgrad_sorted_offset(dtype, n_out, K, cin, cout);
-    rc = tc_conv_wgrad(dtype, X, dY, nbr, MapPlan{row_order, tmap, tmask}, static_cast<float*>(workspace), &chunks, n_out, n_in, K, cin, cout, s,
-                       /*inverse_plan=*/false, sorted_rows, presorted);
-    if (rc != ST_OK) return rc;
+    const void* rows = presorted ? static_cast<char*>(workspace) + wgrad_sorted_offset(dtype, n_out, K, cin, cout) : dY;
+    rc = tc_conv_wgrad(dtype, X, rows, nbr, MapPlan{presorted ? nullptr : row_order, tmap, tmask}, static_cast<float*>(workspace),
+                       &chunks, n_out, n_in, K, cin, cout, s, dW);
+    if (rc != ST_OK || chunks == 0) return rc;
     return reduce_partials(dtype, static_cast<const float*>(workspace), chunks, (int64_t)K * cin * cout, dW, s);
   }
   StoredMap map{nbr, K};
@@ -310,7 +311,7 @@ int st_conv_wgrad_planned_presorted(int dtype, const void* X, const void* dY, co
 
 int64_t st_conv_wgrad_inverse_workspace_bytes(int dtype, int64_t n_in, int K, int cin, int cout) {
   if (n_in < 0 || K < 1 || cin < 1 || cout < 1) return 256;
-  return align_up(tc_wgrad_partial_bytes(dtype, n_in, K, cin, cout), 256) + 256;
+  return align_up(tc_wgrad_planned_bytes(dtype, n_in, K, cin, cout), 256) + 256;
 }
 
 int st_conv_wgrad_inverse_planned(int dtype, const void* X, const void* dY, const int32_t* row_order, const int32_t* tmap,
@@ -333,10 +334,8 @@ int st_conv_wgrad_inverse_planned(int dtype, const void* X, const void* dY, cons
   }
   cudaStream_t s = (cudaStream_t)stream;
   int chunks = 0;
-  rc = tc_conv_wgrad(dtype, X, dY, nullptr, MapPlan{row_order, tmap, tmask}, static_cast<float*>(workspace), &chunks, n_in,
-                     n_out, K, cin, cout, s, true);
-  if (rc != ST_OK) return rc;
-  return reduce_partials(dtype, static_cast<const float*>(workspace), chunks, (int64_t)K * cin * cout, dW, s);
+  return tc_conv_wgrad(dtype, X, dY, nullptr, MapPlan{row_order, tmap, tmask}, static_cast<float*>(workspace), &chunks, n_in,
+                       n_out, K, cin, cout, s, dW, true);
 }
 
 int st_conv_wgrad(int dtype, const void* X, const void* dY, const int32_t* nbr, void* dW, int64_t n_in, int64_t n_out,

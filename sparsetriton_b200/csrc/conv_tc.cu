@@ -13,6 +13,7 @@
 // neighbour map or the coordinate hash table probed on the fly (the Map template argument).
 // Stored maps that come with a tile plan run on the TMA-fed kernels of conv_tc_plan.cuh; the kernels in
 // this file are their cp.async counterparts (hash on the fly, maps without a plan, unaligned tensors).
+#include <algorithm>
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
 
@@ -801,11 +802,10 @@ struct WgradParams {
   int ci_blk;            // input channels per CTA (MMA N)
   int n_ciblk, n_coblk;
   int a_slot_bytes, b_slot_bytes, b_slots;
-  int quad;              // planned_wgrad_kernel: offsets per shared-memory slot (b_slots counts such slots)
   int a_slots;           // planned_wgrad_kernel: depth of the tile-operand ring
+  int weight_a, weight_b;  // planned_wgrad_kernel: what a tile and an offset of a tile cost, in column blocks fetched
+  int32_t* cta_table;    // planned_wgrad_kernel: first CTA of every (offset group, output block, input block), and the total
   int swap;              // planned_wgrad_kernel: 1 = the plan is the INVERSE map's (tile operand X, gathered operand dY)
-  int dense_tiles;       // planned_wgrad_kernel: 1 = the tile operand's rows lie in tile order (a copy permuted by `order`,
-                         // or no `order` at all): a tile is one 2-D box per column block instead of 32 row gathers
   int tmem_cols;
   uint32_t idesc_base;   // everything but N
 };
@@ -1118,9 +1118,6 @@ static bool g_tma_enabled = true;
 
 void tc_set_tma(bool on) { g_tma_enabled = on; }
 
-static bool g_dense_tiles = true;
-void tc_set_dense_tiles(bool on) { g_dense_tiles = on; }
-
 bool tc_supported(int dtype, int c_red, int c_acc) {
   if (!g_tc_enabled) return false;
   if (dtype != ST_F32 && dtype != ST_F16 && dtype != ST_BF16) return false;
@@ -1410,6 +1407,7 @@ static bool plan_wgrad(WgradPlan* plan, int dtype, int64_t n_rows, int K, int ci
   p.group = 512 / p.ci_blk;
   if (p.group > 32) p.group = 32;
   if (p.group > K) p.group = K;
+  while (K > 32 && (p.group & (p.group - 1))) --p.group;       // a group's bits come from one word of the tile mask
   p.n_kgroups = (K + p.group - 1) / p.group;
   // (Equal shares, 7 + 7 + 7 + 6 offsets instead of 8 + 8 + 8 + 3, measured slower: every group then loads the
   // dY tile of nearly every row tile, and the kernel is bound by what the copy engine moves, not by the longest CTA.)
@@ -1522,93 +1520,68 @@ static void launch_permute_rows(const void* src, const int32_t* order, int64_t n
   note_launches(1);
 }
 
-// The copy pass pays for itself when a tile is fetched by four CTAs or more (offset groups x channel blocks); with two
-// groups (32 input channels: 16 offsets per group) it only adds its own cost.
-static bool wgrad_copy_pays(const tc::WgradParams& p) { return p.n_kgroups * p.n_ciblk * p.n_coblk >= 4; }
+// Shape of planned_wgrad_kernel for a layer (on top of plan_wgrad).
+static bool plan_wgrad_planned(WgradPlan* plan, int dtype, int64_t n_rows, int K, int cin, int cout, bool swap) {
+  if (!plan_wgrad(plan, dtype, n_rows, K, cin, cout)) return false;
+  tc::WgradParams& p = plan->p;
+  p.swap = swap ? 1 : 0;
+  // few tiles: smaller groups of offsets, so that there is work for every SM
+  while (p.group > 4 && p.n_tiles * p.n_kgroups * p.n_coblk * p.n_ciblk < sm_count()) {
+    p.group = K > 32 ? p.group / 2 : (p.group + 1) / 2;
+    p.n_kgroups = (K + p.group - 1) / p.group;
+  }
+  if (p.n_kgroups > tc::kWgradMaxGroups) return false;
+  p.tmem_cols = 32;
+  while (p.tmem_cols < p.group * p.ci_blk) p.tmem_cols <<= 1;
+  const int m_full = 128 * p.esize / 128 * tc::kABlockBytes;                     // the MMA reads 128 dY channels, present or not
+  const int m_bytes = (std::min(cout, 128) * p.esize + 127) / 128 * tc::kABlockBytes;
+  const int n_bytes = (p.ci_blk * p.esize + 127) / 128 * tc::kABlockBytes;
+  p.a_slot_bytes = swap ? n_bytes : m_bytes;
+  p.b_slot_bytes = swap ? m_full : n_bytes;
+  p.weight_a = p.a_slot_bytes / tc::kABlockBytes;
+  p.weight_b = p.b_slot_bytes / tc::kABlockBytes;
+  const int budget = 222 * 1024 - (int)sizeof(tc::WgradControl3);
+  // three tile slots when six gathered slots are left, else two
+  p.a_slots = (budget - 3 * p.a_slot_bytes) / p.b_slot_bytes >= 6 ? 3 : 2;
+  p.b_slots = std::min((budget - p.a_slots * p.a_slot_bytes) / p.b_slot_bytes, tc::kWgradBSlots3);
+  // what lies behind the last tile slot must be shared memory too
+  if (p.b_slots < 2 || (!swap && p.b_slots * p.b_slot_bytes < m_full - m_bytes)) return false;
+  // One CTA per SM (each writes its accumulators); with many combinations the shares would be too coarse: two.
+  const int combos = p.n_kgroups * p.n_coblk * p.n_ciblk;
+  int64_t ctas = combos * 3 <= sm_count() ? sm_count() : std::max(2 * sm_count(), combos);
+  ctas = std::max<int64_t>(std::min<int64_t>(ctas, p.n_tiles * combos), combos);
+  plan->n_chunks = (int)ctas;
+  plan->smem = (size_t)p.a_slots * p.a_slot_bytes + (size_t)p.b_slots * p.b_slot_bytes + sizeof(tc::WgradControl3) + 1024;
+  return true;
+}
 
-// Tile-plan form: the TMA-fed kernel when both tensors can be described to the copy engine and two
-// slots fit, else the cp.async producers of wgrad_kernel over the same plan.  `sorted_rows`: scratch for a copy of
-// the tile operand in tile order (n_rows x cout elements), or null.
-static int launch_wgrad_planned(WgradPlan& plan, const tc::PlannedRows& map, cudaStream_t stream, void* sorted_rows,
-                                bool presorted) {
+static int64_t wgrad_table_bytes(const tc::WgradParams& p) {
+  return ((int64_t)(p.n_kgroups * p.n_coblk * p.n_ciblk + 1) * 4 + 255) / 256 * 256;
+}
+
+// Workspace of the tile-plan form: the division of the CTAs, then a block of partial sums per CTA.
+int64_t tc_wgrad_planned_bytes(int dtype, int64_t n_rows, int K, int cin, int cout) {
+  int64_t most = 0;
+  for (bool swap : {false, true}) {
+    WgradPlan plan;
+    if (!plan_wgrad_planned(&plan, dtype, n_rows, K, cin, cout, swap)) continue;
+    const tc::WgradParams& p = plan.p;
+    most = std::max(most, wgrad_table_bytes(p) + (int64_t)plan.n_chunks * p.group * p.ci_blk * std::min(cout, 128) * 4);
+  }
+  return most;
+}
+
+static bool aligned16(const void* a) { return (reinterpret_cast<uintptr_t>(a) & 15) == 0; }
+
+// Tile-plan form: the product and the sum of its partials.  Rows of whole 16-byte pieces only.
+static int launch_wgrad_planned(WgradPlan& plan, const tc::PlannedRows& map, int dtype, void* dw, cudaStream_t stream) {
   tc::WgradParams& p = plan.p;
-  if (p.swap) {
-    // ring 1 holds X tiles (ci_blk wide), ring 2 the gathered dY rows (128 output channels wide)
-    const int t = p.a_slot_bytes;
-    p.a_slot_bytes = p.b_slot_bytes;
-    p.b_slot_bytes = t;
-  }
-  // Shared memory: a ring of dY tiles and a ring of X-row slots of `quad` offsets each.  Two shapes, chosen by
-  // measurement: rows of one 128-byte line travel four offsets to a slot, two slots, indices loaded as the
-  // task comes up; wider rows (two lines, 128 or more 16-bit channels) travel one offset to a slot with three
-  // dY tiles in flight and the indices loaded ahead.
-  const bool wide = p.b_slot_bytes >= 2 * tc::kABlockBytes;
-  int a_slots = wide ? 3 : 2, quad = wide ? 1 : tc::kProducerWarps, ahead = wide ? 2 : 0, b_cap = wide ? tc::kWgradBSlots3 : 4;
-#ifdef ST_TC_PROFILE
-  {
-    const char* e = getenv("ST_TC_QUAD");
-    if (e && atoi(e) >= 1 && atoi(e) <= tc::kProducerWarps) quad = atoi(e);
-    const char* f = getenv("ST_TC_ASLOTS");
-    if (f && atoi(f) >= 2 && atoi(f) <= tc::kWgradASlots3) a_slots = atoi(f);
-    const char* g = getenv("ST_TC_AHEAD");
-    if (g) ahead = atoi(g);
-    const char* h = getenv("ST_TC_BCAP");
-    if (h && atoi(h) >= 2 && atoi(h) <= tc::kWgradBSlots3) b_cap = atoi(h);
-  }
-#endif
-  if (quad > p.group) quad = p.group;
-  int budget = 222 * 1024 - a_slots * p.a_slot_bytes - (int)sizeof(tc::WgradControl3);
-  while (a_slots > 2 && budget < 2 * quad * p.b_slot_bytes) {
-    --a_slots;
-    budget += p.a_slot_bytes;
-  }
-  while (quad > 1 && budget < 2 * quad * p.b_slot_bytes) --quad;
-  CUtensorMap x_desc, dy_desc, tile_box_desc;
-  memset(&x_desc, 0, sizeof(x_desc));
-  memset(&dy_desc, 0, sizeof(dy_desc));
-  memset(&tile_box_desc, 0, sizeof(tile_box_desc));
-  const int dtype = p.esize == 4 ? ST_F32 : ST_BF16;      // element size is all the copy engine needs to know
-  const bool tma = g_tma_enabled && budget >= 2 * quad * p.b_slot_bytes && p.n_src > 0 &&
-                   make_gather_desc(&x_desc, p.x, p.swap ? p.n_rows : p.n_src, p.cin, p.esize, dtype, p.esize == 4) &&
-                   make_gather_desc(&dy_desc, p.dy, p.swap ? p.n_src : p.n_rows, p.cout, p.esize, dtype, p.esize == 4);
-  // The dY tile of a step is 128 rows picked through `order`: 32 row gathers per 128-byte column block, and every
-  // offset group (and input-channel block) of a row chunk fetches it again.  With the rows copied into tile order once
-  // (one streaming pass) a tile is a dense box, which the copy engine moves 2.3x faster.
-  // `presorted`: the caller made that copy already (tc_wgrad_sort_rows, typically on another stream beside the
-  // feature gradient).
-  p.dense_tiles = 0;
-  if (tma && !p.swap && g_dense_tiles &&
-      (p.order == nullptr || (sorted_rows != nullptr && (presorted || wgrad_copy_pays(p)))) &&
-      (p.cout * p.esize) % 16 == 0) {
-    const void* tiles = p.dy;
-    if (p.order) {
-      if (!presorted) launch_permute_rows(p.dy, p.order, p.n_rows, p.cout * p.esize / 16, sorted_rows, stream);
-      tiles = sorted_rows;
-    }
-    if (make_weight_desc(&tile_box_desc, tiles, p.n_rows, p.cout, p.esize, dtype, tc::kTileM, p.esize == 4)) p.dense_tiles = 1;
-  }
-  if (!tma) {
-    if (p.swap) {
-      set_error("tc wgrad over the inverse plan needs the TMA kernels (16-byte aligned tensors, st_set_tma(1))");
-      return ST_ERR_UNSUPPORTED;
-    }
-    return launch_wgrad(plan, map, stream);
-  }
-  p.quad = quad;
-  p.a_slots = a_slots;
-  int slots = budget / (quad * p.b_slot_bytes);
-#ifdef ST_TC_PROFILE
-  {
-    const char* e = getenv("ST_TC_BSLOTS");
-    if (e && atoi(e) >= 2 && atoi(e) <= slots) slots = atoi(e);
-  }
-#endif
-  p.b_slots = slots > b_cap ? b_cap : slots;
-  const size_t smem = (size_t)a_slots * p.a_slot_bytes + (size_t)p.b_slots * quad * p.b_slot_bytes + sizeof(tc::WgradControl3) + 1024;
-  auto kernel = ahead == 0 ? tc::planned_wgrad_kernel<0> : (ahead == 2 ? tc::planned_wgrad_kernel<2> : tc::planned_wgrad_kernel<4>);
+  p.cta_table = reinterpret_cast<int32_t*>(p.partial);
+  p.partial = reinterpret_cast<float*>(reinterpret_cast<char*>(p.partial) + wgrad_table_bytes(p));
+  auto kernel = p.esize == 4 ? tc::planned_wgrad_kernel<4> : tc::planned_wgrad_kernel<2>;
   static bool configured[kMaxDevices] = {};
   if (!configured[current_device()]) {
-    for (auto k : {tc::planned_wgrad_kernel<0>, tc::planned_wgrad_kernel<2>, tc::planned_wgrad_kernel<4>}) {
+    for (auto k : {tc::planned_wgrad_kernel<2>, tc::planned_wgrad_kernel<4>}) {
       cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
       if (e != cudaSuccess) {
         set_error("tc planned wgrad: cannot raise the dynamic shared memory limit: %s", cudaGetErrorString(e));
@@ -1617,9 +1590,15 @@ static int launch_wgrad_planned(WgradPlan& plan, const tc::PlannedRows& map, cud
     }
     configured[current_device()] = true;
   }
-  dim3 grid((unsigned)plan.n_chunks, (unsigned)p.n_kgroups, (unsigned)(p.n_coblk * p.n_ciblk));
-  kernel<<<grid, tc::kThreads, smem, stream>>>(p, map, x_desc, dy_desc, tile_box_desc);
-  note_launches(1);
+  kernel<<<(unsigned)plan.n_chunks, tc::kWgrad3Threads, plan.smem, stream>>>(p, map);
+  const unsigned blocks = (unsigned)(((int64_t)p.K * p.cin * (p.cout / 4) + 31) / 32);
+  if (dtype == ST_F32)
+    tc::wgrad_sum_kernel<float><<<blocks, 256, 0, stream>>>(p, static_cast<float*>(dw));
+  else if (dtype == ST_F16)
+    tc::wgrad_sum_kernel<__half><<<blocks, 256, 0, stream>>>(p, static_cast<__half*>(dw));
+  else
+    tc::wgrad_sum_kernel<__nv_bfloat16><<<blocks, 256, 0, stream>>>(p, static_cast<__nv_bfloat16*>(dw));
+  note_launches(2);
   return check_launch("tc planned wgrad");
 }
 
@@ -1632,40 +1611,45 @@ static bool prepare_wgrad(WgradPlan* plan, int dtype, const void* x, const void*
   plan->p.x = x;
   plan->p.dy = dy;
   plan->p.order = nullptr;
-  plan->p.quad = 1;
   plan->p.a_slots = 2;
   plan->p.swap = 0;
-  plan->p.dense_tiles = 0;
   plan->p.partial = partial;
   plan->p.n_src = n_src;
   return true;
 }
 
 int tc_conv_wgrad(int dtype, const void* x, const void* dy, const int32_t* map, const MapPlan& rows, float* partial,
-                  int* n_chunks_out, int64_t n_rows, int64_t n_src, int K, int cin, int cout, cudaStream_t stream,
-                  bool inverse_plan, void* sorted_rows, bool presorted) {
+                  int* n_chunks_out, int64_t n_rows, int64_t n_src, int K, int cin, int cout, cudaStream_t stream, void* dw,
+                  bool inverse_plan) {
   WgradPlan plan;
+  const bool has_plan = rows.tmap && rows.tmask;
+  if (has_plan && g_tma_enabled && aligned16(x) && aligned16(dy) && n_src > 0 && n_src <= 0x7FFFFFFFll &&
+      plan_wgrad_planned(&plan, dtype, n_rows, K, cin, cout, inverse_plan)) {
+    plan.p.x = x;
+    plan.p.dy = dy;
+    plan.p.order = rows.order;
+    plan.p.partial = partial;
+    plan.p.n_src = n_src;
+    *n_chunks_out = 0;
+    return launch_wgrad_planned(plan, tc::PlannedRows{rows.tmap, rows.tmask, K, (K + 31) / 32}, dtype, dw, stream);
+  }
+  if (inverse_plan) {
+    set_error("tc wgrad over the inverse plan needs a tile plan and 16-byte aligned tensors (st_set_tma(1))");
+    return has_plan ? ST_ERR_UNSUPPORTED : ST_ERR_ARG;
+  }
   if (!prepare_wgrad(&plan, dtype, x, dy, partial, n_rows, n_src, K, cin, cout)) return ST_ERR_UNSUPPORTED;
   plan.p.order = rows.order;
-  plan.p.swap = inverse_plan ? 1 : 0;
-  if (inverse_plan && !(rows.tmap && rows.tmask)) {
-    set_error("tc wgrad: the inverse form needs a tile plan");
-    return ST_ERR_ARG;
-  }
-  int rc;
-  if (rows.tmap && rows.tmask)
-    rc = launch_wgrad_planned(plan, tc::PlannedRows{rows.tmap, rows.tmask, K, (K + 31) / 32}, stream, sorted_rows,
-                              presorted);
-  else
-    rc = launch_wgrad(plan, tc::StoredRows{map, K}, stream);
+  const int rc = has_plan ? launch_wgrad(plan, tc::PlannedRows{rows.tmap, rows.tmask, K, (K + 31) / 32}, stream)
+                          : launch_wgrad(plan, tc::StoredRows{map, K}, stream);
   *n_chunks_out = plan.n_chunks;
   return rc;
 }
 
+// A layer whose tiles of dY several CTAs fetch: four or more (offset group, channel block) combinations.
 bool tc_wgrad_sorts_rows(int dtype, int64_t n_rows, int K, int cin, int cout) {
   WgradPlan plan;
-  if (!g_tma_enabled || !g_dense_tiles || !plan_wgrad(&plan, dtype, n_rows, K, cin, cout)) return false;
-  return wgrad_copy_pays(plan.p) && (plan.p.cout * plan.p.esize) % 16 == 0;
+  if (!g_tma_enabled || !plan_wgrad(&plan, dtype, n_rows, K, cin, cout)) return false;
+  return plan.p.n_kgroups * plan.p.n_ciblk * plan.p.n_coblk >= 4 && (plan.p.cout * plan.p.esize) % 16 == 0;
 }
 
 int tc_wgrad_sort_rows(int dtype, const void* dy, const int32_t* order, int64_t n_rows, int cout, void* sorted,

@@ -15,7 +15,6 @@ bool tc_supported(int dtype, int c_red, int c_acc);
 void tc_set_enabled(bool on);
 // Process-wide switch: when off, products over a tile plan run their cp.async forms instead of the TMA-fed ones.
 void tc_set_tma(bool on);
-void tc_set_dense_tiles(bool on);
 
 // OUT[r,:] = sum_k IN[map[r,k],:] . B_k over a stored (n_rows, K) map.
 //   w_transposed = false: B_k = W[k]   with W (K, c_red, c_acc)   (forward)
@@ -60,13 +59,15 @@ int tc_conv_wgrad_hashfly(int dtype, const void* x, const void* dy, const HashFl
 // Tensor-core weight gradient: fills fp32 partials (n_chunks, K, cin, cout) that the caller reduces.
 bool tc_wgrad_supported(int dtype, int64_t n_rows, int K, int cin, int cout);
 int64_t tc_wgrad_partial_bytes(int dtype, int64_t n_rows, int K, int cin, int cout);
+// Over a tile plan the whole weight gradient is made, into dw, and *n_chunks_out is 0 (nothing is left to reduce).
 // inverse_plan: `plan` is the tile plan of the INVERSE map; then n_rows counts the rows of x (the plan's rows) and
 // n_src the rows of dy (the rows the plan's entries name).
 int tc_conv_wgrad(int dtype, const void* x, const void* dy, const int32_t* map, const MapPlan& plan, float* partial,
-                  int* n_chunks_out, int64_t n_rows, int64_t n_src, int K, int cin, int cout, cudaStream_t stream,
-                  bool inverse_plan = false, void* sorted_rows = nullptr, bool presorted = false);
-// Whether tc_conv_wgrad over a tile plan with a row order would copy dY into tile order (into `sorted_rows`), and that
-// copy alone; with it made beforehand, tc_conv_wgrad takes presorted = true.
+                  int* n_chunks_out, int64_t n_rows, int64_t n_src, int K, int cin, int cout, cudaStream_t stream, void* dw,
+                  bool inverse_plan = false);
+int64_t tc_wgrad_planned_bytes(int dtype, int64_t n_rows, int K, int cin, int cout);
+// Whether a copy of dY in tile order is offered for this layer (st_conv_wgrad_presort), and that copy alone; with it made
+// beforehand, tc_conv_wgrad takes the copy as dy and no order.
 bool tc_wgrad_sorts_rows(int dtype, int64_t n_rows, int K, int cin, int cout);
 int tc_wgrad_sort_rows(int dtype, const void* dy, const int32_t* order, int64_t n_rows, int cout, void* sorted,
                        cudaStream_t stream);

@@ -88,13 +88,13 @@ __device__ __forceinline__ void walk_super_tiles(const Params2& p, const Planned
   }
 }
 
-// A warp's 32 rows of a stage: 2^kLpr lanes share a row (16 bytes each).  All row numbers are exchanged before the first
-// copy: a shuffle behind a cp.async in the memory pipe waits for it (450 cycles per copy when they alternated).
-template <int kLpr>
+// A warp's kRows (32 or 8) rows of one 128-byte column block: 2^kLpr lanes share a row (16 bytes each).  All row numbers are
+// exchanged before the first copy.  kAtom32: the 128-byte swizzle with 32-byte atoms, else the plain one.
+template <int kLpr, int kRows, bool kAtom32>
 __device__ __forceinline__ void fetch_rows(uint32_t dst, int row0, int idx, const char* col, int pitch, int64_t n_src, int chunks,
                                            int lane) {
-  constexpr int kRowsPer = 32 >> kLpr, kN = 1 << kLpr;
-  const int c = lane & (kN - 1), r_lane = lane >> kLpr;
+  constexpr int kRowsPer = 32 >> kLpr, kN = kRows > kRowsPer ? kRows / kRowsPer : 1;
+  const int c = lane & ((1 << kLpr) - 1), r_lane = lane >> kLpr;
   int src[kN];
 #pragma unroll
   for (int i = 0; i < kN; ++i) src[i] = __shfl_sync(0xFFFFFFFFu, idx, i * kRowsPer + r_lane);
@@ -103,10 +103,19 @@ __device__ __forceinline__ void fetch_rows(uint32_t dst, int row0, int idx, cons
   for (int i = 0; i < kN; ++i) {
     const bool have = (uint32_t)src[i] < (uint32_t)n_src;                      // "-1" and rows past the source: zeros
     const int row = row0 + i * kRowsPer + r_lane;
-    if (c < chunks)
-      cp_async16(dst + (uint32_t)row * 128u + ((uint32_t)swz16(c, row) << 4),
+    if (c < chunks && (kRows >= kRowsPer || r_lane < kRows))
+      cp_async16(dst + (uint32_t)row * 128u + ((uint32_t)(kAtom32 ? swz32(c, row) : swz16(c, row)) << 4),
                  col + (have ? (size_t)(uint32_t)src[i] * (uint32_t)pitch : 0), have ? 16u : 0u);
   }
+}
+// ... of a row block of `bytes` (a multiple of 16, at most 128) bytes.
+template <int kRows, bool kAtom32>
+__device__ __forceinline__ void fetch_block(uint32_t dst, int row0, int idx, const char* col, int pitch, int64_t n_src, int bytes,
+                                            int lane) {
+  const int chunks = bytes >> 4;
+  if (chunks > 4) fetch_rows<3, kRows, kAtom32>(dst, row0, idx, col, pitch, n_src, chunks, lane);
+  else if (chunks > 2) fetch_rows<2, kRows, kAtom32>(dst, row0, idx, col, pitch, n_src, chunks, lane);
+  else fetch_rows<1, kRows, kAtom32>(dst, row0, idx, col, pitch, n_src, chunks, lane);
 }
 
 template <int ESIZE>
@@ -165,12 +174,8 @@ __global__ void __launch_bounds__(kGather3Threads, 1) planned_gather_kernel(cons
     auto run = [&]() {
       ok = mbar_wait_all(smem_u32(&ctl->a_empty[pend_stage]), pend_parity ^ 1u, abort_flag, 31);
       if (!ok) return;
-      const int chunks = min(128, red_bytes - pend_kb * 128) >> 4;             // 16-byte pieces of a row: 2, 4, 6 or 8
-      const uint32_t dst = a_ring + (uint32_t)pend_stage * kABlockBytes;
-      const char* col = in + pend_kb * 128;
-      if (chunks > 4) fetch_rows<3>(dst, row0, pend_idx, col, red_bytes, p.n_src, chunks, lane);
-      else if (chunks > 2) fetch_rows<2>(dst, row0, pend_idx, col, red_bytes, p.n_src, chunks, lane);
-      else fetch_rows<1>(dst, row0, pend_idx, col, red_bytes, p.n_src, chunks, lane);
+      fetch_block<32, false>(a_ring + (uint32_t)pend_stage * kABlockBytes, row0, pend_idx, in + pend_kb * 128, red_bytes, p.n_src,
+                         min(128, red_bytes - pend_kb * 128), lane);
       cp_async_commit();
       cp_async_wait_group<1>();                               // the share before this one has landed: announce it
       __syncwarp();
@@ -383,23 +388,28 @@ __global__ void __launch_bounds__(kGather3Threads, 1) planned_gather_kernel(cons
 
 
 // =================================================================================================
-// Weight gradient over a stored map in tile-plan form, fed by TMA.
+// Weight gradient over a stored map in tile-plan form.
 //
 //   dW[k][ci][co] = sum_r  X[tmap(r, k)][ci] * dY[order[r]][co]
 //
-// Same decomposition as wgrad_kernel (a CTA owns a chunk of row tiles, a group of G offsets whose G
-// accumulators fill TMEM, a block of output channels and one of input channels; fp32 partials per
-// chunk), but:
-//   - the tile's mask says which offsets of the group have any neighbour in the tile; both the
-//     producers and the MMA thread read it, so no step descriptors travel through shared memory;
-//   - the dY tile and the gathered X rows arrive by tile::gather4 (rows of dY through `order`, rows
-//     of X through the tile's index lines);
-//   - up to Q offsets share one shared-memory slot and one mbarrier (producer warp q fetches the
-//     rows of the q-th of them), so the MMA thread waits and commits once per Q x 8 (16) MMAs.
-// Every producer warp arrives on every barrier (see planned_gather_kernel).
+// A CTA owns a group of G offsets (G accumulators fill TMEM), a block of output and one of input channels, and a share
+// of the row tiles.  Per tile that has an offset of the group it brings in the tile operand (128 rows of dY, picked through
+// `order`) once and the gathered operand (128 rows of X through the tile's index line) per offset; both come with 16-byte
+// cp.async from 16 warps, as in planned_gather_kernel, through two rings.  With p.swap the plan is the INVERSE map's: the
+// tile operand is X and the gathered one dY.
+//
+// How the CTAs are shared out: an odd kernel's centre offset occurs in every tile of a submanifold layer and the others in
+// a tenth to a third of them, so equal shares left the centre's group with half of the work on a quarter of the CTAs.
+// Every CTA therefore weighs the groups itself (stages over the tile masks, from L2, at most 4096 tiles looked at: 2-3 us)
+// and all come to the same division, one or more CTAs per (group, channel blocks) in proportion.  One CTA per SM: every
+// CTA writes its accumulators (up to 256 KB of fp32 partial sums), which a second kernel adds in a fixed order.
 // =================================================================================================
 constexpr int kWgradASlots3 = 4;
 constexpr int kWgradBSlots3 = 12;
+constexpr int kWgradRowWarp0 = kMmaWarp + 1;
+constexpr int kWgrad3Threads = (kWgradRowWarp0 + kRowGroups * kRowGroupWarps) * 32;
+constexpr int kWgradMaxGroups = 96;                             // ST_MAX_KVOL offsets in groups of four, and some
+constexpr int64_t kWgradWeighed = 4096;                         // tiles looked at to weigh the groups
 
 struct __align__(8) WgradControl3 {
   unsigned long long a_full[kWgradASlots3], a_empty[kWgradASlots3];
@@ -408,57 +418,56 @@ struct __align__(8) WgradControl3 {
   uint32_t touched;
   uint32_t tmem_base;
   int abort_flag;
+  int combo, first_cta, n_ctas;
+  uint32_t weight[kWgradMaxGroups];
 };
 
-template <int kAhead>
-__global__ void __launch_bounds__(kThreads, 1) planned_wgrad_kernel(const WgradParams p, const PlannedRows map,
-                                                                    const __grid_constant__ CUtensorMap x_desc,
-                                                                    const __grid_constant__ CUtensorMap dy_desc,
-                                                                    const __grid_constant__ CUtensorMap tile_box_desc) {
+// f(tile, mask) for every tile of this CTA that has an offset of its group, 32 masks loaded at a time.
+template <typename F>
+__device__ __forceinline__ void walk_tiles(const WgradParams& p, const PlannedRows& map, int64_t first, int64_t step, int word,
+                                           int shift, uint32_t group_bits, int lane, F&& f) {
+  auto load = [&](int64_t t0) {
+    const int64_t tile = t0 + lane * step;
+    return tile < p.n_tiles ? (__ldg(map.tmask + tile * map.MW + word) >> shift) & group_bits : 0u;
+  };
+  uint32_t next = load(first);
+  for (int64_t t0 = first; t0 < p.n_tiles; t0 += 32 * step) {
+    const uint32_t mine = next;
+    next = load(t0 + 32 * step);
+    uint32_t live = __ballot_sync(0xFFFFFFFFu, mine != 0u);
+    while (live) {
+      const int l = __ffs(live) - 1;
+      live &= live - 1;
+      if (!f(t0 + l * step, __reduce_or_sync(0xFFFFFFFFu, lane == l ? mine : 0u))) return;
+    }
+  }
+}
+
+template <int ESIZE>
+__global__ void __launch_bounds__(kWgrad3Threads, 1) planned_wgrad_kernel(const WgradParams p, const PlannedRows map) {
   extern __shared__ unsigned char smem_raw[];
   const uint32_t raw = smem_u32(smem_raw);
   const uint32_t base = (raw + 1023u) & ~1023u;
   unsigned char* base_ptr = smem_raw + (base - raw);
   const uint32_t a_ring = base;
   const uint32_t b_ring = base + (uint32_t)p.a_slots * (uint32_t)p.a_slot_bytes;
-  const uint32_t quad_bytes = (uint32_t)p.quad * (uint32_t)p.b_slot_bytes;
-  WgradControl3* ctl = reinterpret_cast<WgradControl3*>(base_ptr + (size_t)p.a_slots * p.a_slot_bytes + (size_t)p.b_slots * quad_bytes);
+  WgradControl3* ctl = reinterpret_cast<WgradControl3*>(base_ptr + (size_t)p.a_slots * p.a_slot_bytes +
+                                                        (size_t)p.b_slots * p.b_slot_bytes);
   volatile int* abort_flag = &ctl->abort_flag;
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = __shfl_sync(0xFFFFFFFFu, (int)(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;
+  auto bits_of = [&](int kgroup) {
+    const int n = min(p.group, p.K - kgroup * p.group);
+    return n >= 32 ? 0xFFFFFFFFu : ((1u << n) - 1u);
+  };
 
-  // work item of this CTA
-  const int chunk = blockIdx.x;
-  const int kgroup = blockIdx.y;
-  const int coblk = blockIdx.z / p.n_ciblk, ciblk = blockIdx.z % p.n_ciblk;
-  const int k_first = kgroup * p.group;
-  const int g_count = min(p.group, p.K - k_first);
-  const int co0 = coblk * 128, co_cnt = min(128, p.cout - co0);
-  const int ci0 = ciblk * p.ci_blk, ci_cnt = min(p.ci_blk, p.cin - ci0);
-  // The chunk takes every gridDim.x-th tile: in sorted row order the number of occupied offsets grows
-  // along the rows, so contiguous ranges of tiles would be very unequal pieces of work.
-  const int64_t tile_begin = chunk, tile_end = p.n_tiles, tile_step = gridDim.x;
-  const int word = k_first >> 5, shift = k_first & 31;
-  const uint32_t group_bits = g_count >= 32 ? 0xFFFFFFFFu : ((1u << g_count) - 1u);
-  const int per_line = 128 / p.esize;                       // elements of one 128-byte line
-  // The per-tile operand (ring 1, rows taken through `order`) and the per-offset operand (ring 2, rows taken
-  // through the plan's index lines).  Over the forward map the tile operand is dY (M side of the product) and
-  // the gathered one X (N side); with p.swap the kernel walks the plan of the INVERSE map instead: the tile
-  // operand is X, the gathered one dY, and the MMA takes its A operand from ring 2 and its B operand from ring 1.
-  const int m_blocks = (co_cnt * p.esize + 127) >> 7;       // 128-byte column blocks of dY rows
-  const int n_blocks = (ci_cnt * p.esize + 127) >> 7;       // ... of X rows
-  const int a_blocks = p.swap ? n_blocks : m_blocks;        // blocks of the tile operand
-  const int b_blocks = p.swap ? m_blocks : n_blocks;        // blocks of the gathered operand
-  const CUtensorMap* tile_desc = p.swap ? &x_desc : &dy_desc;
-  const CUtensorMap* gath_desc = p.swap ? &dy_desc : &x_desc;
-  const int tile_col0 = p.swap ? ci0 : co0, gath_col0 = p.swap ? co0 : ci0;
-
+  for (int g = threadIdx.x; g < p.n_kgroups; g += kWgrad3Threads) ctl->weight[g] = 0;
   if (threadIdx.x == 0) {
     for (int s = 0; s < p.a_slots; ++s) {
-      mbar_init(smem_u32(&ctl->a_full[s]), kProducerWarps);
+      mbar_init(smem_u32(&ctl->a_full[s]), kRowGroups * kRowGroupWarps);
       mbar_init(smem_u32(&ctl->a_empty[s]), 1);
     }
     for (int s = 0; s < p.b_slots; ++s) {
-      mbar_init(smem_u32(&ctl->b_full[s]), kProducerWarps);
+      mbar_init(smem_u32(&ctl->b_full[s]), kRowGroupWarps);
       mbar_init(smem_u32(&ctl->b_empty[s]), 1);
     }
     mbar_init(smem_u32(&ctl->acc_full), 2);
@@ -474,317 +483,207 @@ __global__ void __launch_bounds__(kThreads, 1) planned_wgrad_kernel(const WgradP
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = ctl->tmem_base;
-  const bool base32 = p.esize == 4;                 // 32-bit elements: 128-byte swizzle with 32-byte atoms
+  // ---- which work is this CTA's: weigh the groups, divide gridDim.x CTAs among the combinations
+  const int n_blocks2 = p.n_coblk * p.n_ciblk, n_combos = p.n_kgroups * n_blocks2;
+  {
+    const int64_t stride = p.n_tiles > kWgradWeighed ? p.n_tiles / kWgradWeighed : 1;
+    for (int g = 0; g < p.n_kgroups; ++g) {
+      const int k0 = g * p.group;
+      uint32_t sum = 0;
+      for (int64_t t = threadIdx.x * stride; t < p.n_tiles; t += kWgrad3Threads * stride) {
+        const uint32_t m = (__ldg(map.tmask + t * map.MW + (k0 >> 5)) >> (k0 & 31)) & bits_of(g);
+        if (m) sum += (uint32_t)p.weight_a + (uint32_t)__popc(m) * (uint32_t)p.weight_b;
+      }
+      sum = __reduce_add_sync(0xFFFFFFFFu, sum);
+      if (lane == 0 && sum) atomicAdd(&ctl->weight[g], sum);
+    }
+    __syncthreads();
+    uint64_t total = 0;
+    for (int g = 0; g < p.n_kgroups; ++g) total += ctl->weight[g];
+    if (total == 0) total = 1;
+    auto start_of = [&](int combo) {                           // first CTA of a combination: one each, the rest by weight
+      uint64_t before = 0;
+      const int g = combo / n_blocks2;
+      for (int i = 0; i < g; ++i) before += (uint64_t)ctl->weight[i] * n_blocks2;
+      if (g < p.n_kgroups) before += (uint64_t)ctl->weight[g] * (combo - g * n_blocks2);
+      return combo + (int)(before * (uint64_t)(gridDim.x - n_combos) / (total * n_blocks2));
+    };
+    for (int c = threadIdx.x; c < n_combos; c += kWgrad3Threads) {
+      // with no neighbour anywhere the last combination takes what is left
+      const int first = start_of(c), end = c + 1 == n_combos ? (int)gridDim.x : start_of(c + 1);
+      if ((int)blockIdx.x >= first && (int)blockIdx.x < end) {
+        ctl->combo = c;
+        ctl->first_cta = first;
+        ctl->n_ctas = end - first;
+      }
+      if (blockIdx.x == 0) {
+        p.cta_table[c] = first;
+        if (c + 1 == n_combos) p.cta_table[n_combos] = end;
+      }
+    }
+    __syncthreads();
+  }
+  const int combo = __shfl_sync(0xFFFFFFFFu, ctl->combo, 0);
+  const int kgroup = combo / n_blocks2;
+  const int coblk = combo % n_blocks2 / p.n_ciblk, ciblk = combo % p.n_ciblk;
+  const int64_t tile_begin = blockIdx.x - __shfl_sync(0xFFFFFFFFu, ctl->first_cta, 0);
+  const int64_t tile_step = __shfl_sync(0xFFFFFFFFu, ctl->n_ctas, 0);       // neighbouring tiles are alike: deal them out
+  const int k_first = kgroup * p.group;
+  const int g_count = min(p.group, p.K - k_first);
+  const int co0 = coblk * 128, co_cnt = min(128, p.cout - co0);
+  const int ci0 = ciblk * p.ci_blk, ci_cnt = min(p.ci_blk, p.cin - ci0);
+  const int word = k_first >> 5, shift = k_first & 31;
+  const uint32_t group_bits = bits_of(kgroup);
+  constexpr bool kBase32 = ESIZE == 4;                      // 32-bit elements: 128-byte swizzle with 32-byte atoms
 
-  auto tile_mask = [&](int64_t tile) { return (__ldg(map.tmask + tile * map.MW + word) >> shift) & group_bits; };
-
-  if (warp >= kFirstProducerWarp) {
-    // =============================================================== producers
-    // The CTA's copies form one sequence of tasks: per tile with an occupied offset, the dY tile (A), then
-    // one slot of X rows per `quad` occupied offsets (B).  Every producer warp walks the whole sequence (it
-    // has to arrive on every barrier) with two cursors: `fetch` runs kAhead tasks in front and loads the
-    // row indices a task needs (a line of `order` or of the plan) into a short register queue, `issue`
-    // waits for the task's slot and starts its copies with indices that have long arrived.  Without the
-    // look-ahead every slot paid one trip to DRAM for its indices before its copies could start.
-    if constexpr (kAhead == 0) {
-      // plain form: each task loads its row indices, waits for its slot and starts its copies
-      const int pw = warp - kFirstProducerWarp;
-      int a_slot = 0, b_slot = 0;
-      uint32_t a_phase = 0, b_phase = 0;
-      bool ok = true;
-      uint32_t m_next = tile_begin < tile_end ? tile_mask(tile_begin) : 0u;
-      for (int64_t tile = tile_begin; tile < tile_end && ok; tile += tile_step) {
-        uint32_t m = m_next;
-        if (tile + tile_step < tile_end) m_next = tile_mask(tile + tile_step);
-        if (!m) continue;
-        // ---- the dY tile: rows order[tile * 128 + r], or one dense box when the rows lie in tile order
-        if (p.dense_tiles) {
-          ok = mbar_wait_all(smem_u32(&ctl->a_empty[a_slot]), a_phase ^ 1u, abort_flag, 35);
-          if (!ok) break;
-          const uint32_t bar = smem_u32(&ctl->a_full[a_slot]);
-          const uint32_t slot_base = a_ring + (uint32_t)a_slot * (uint32_t)p.a_slot_bytes;
-          if (lane == 0) {
-            int mine = 0;
-            for (int b = pw; b < a_blocks; b += kProducerWarps) ++mine;
-            if (mine) mbar_arrive_expect_tx(bar, (uint32_t)mine * kABlockBytes); else mbar_arrive(bar);
-            for (int b = pw; b < a_blocks; b += kProducerWarps)
-              tma_load_2d(slot_base + (uint32_t)b * kABlockBytes, &tile_box_desc, bar, tile_col0 + b * per_line,
-                          (int)(tile * kTileM));
-          }
-          __syncwarp();
-          if (++a_slot == p.a_slots) {
-            a_slot = 0;
-            a_phase ^= 1u;
-          }
-        } else {
-          const int64_t pos = tile * kTileM + 4 * lane;
-          int4 rows;
-          if (p.order) {
-            // the last tile's line may run past the end of `order`: read only what exists
-            rows.x = pos + 0 < p.n_rows ? __ldg(p.order + pos + 0) : -1;
-            rows.y = pos + 1 < p.n_rows ? __ldg(p.order + pos + 1) : -1;
-            rows.z = pos + 2 < p.n_rows ? __ldg(p.order + pos + 2) : -1;
-            rows.w = pos + 3 < p.n_rows ? __ldg(p.order + pos + 3) : -1;
-          } else {
-            rows = make_int4((int)pos, (int)pos + 1, (int)pos + 2, (int)pos + 3);
-          }
-          if (pos + 0 >= p.n_rows) rows.x = -1;
-          if (pos + 1 >= p.n_rows) rows.y = -1;
-          if (pos + 2 >= p.n_rows) rows.z = -1;
-          if (pos + 3 >= p.n_rows) rows.w = -1;
-          ok = mbar_wait_all(smem_u32(&ctl->a_empty[a_slot]), a_phase ^ 1u, abort_flag, 35);
-          if (!ok) break;
-          const uint32_t bar = smem_u32(&ctl->a_full[a_slot]);
-          const uint32_t slot_base = a_ring + (uint32_t)a_slot * (uint32_t)p.a_slot_bytes;
-          // column block b is fetched by warp b % 4
-          int mine = 0;
-          for (int b = pw; b < a_blocks; b += kProducerWarps) ++mine;
-          if (lane == 0) {
-            if (mine) mbar_arrive_expect_tx(bar, (uint32_t)mine * kABlockBytes); else mbar_arrive(bar);
-          }
-          __syncwarp();
-          for (int b = pw; b < a_blocks; b += kProducerWarps)
-            tma_gather4(slot_base + (uint32_t)b * kABlockBytes + (uint32_t)lane * 512u, tile_desc, bar, tile_col0 + b * per_line,
-                        rows.x, rows.y, rows.z, rows.w);
-          if (++a_slot == p.a_slots) {
-            a_slot = 0;
-            a_phase ^= 1u;
-          }
-        }
-        // ---- the gathered X rows, `quad` offsets per slot: warp q fetches the q-th of them
-        while (m && ok) {
-          int my_j = -1;
-          for (int q = 0; q < p.quad && m; ++q) {
-            const int j = __ffs(m) - 1;
-            m &= m - 1;
-            if (q == pw) my_j = j;
-          }
-          int4 idx = make_int4(-1, -1, -1, -1);
-          if (my_j >= 0)
-            idx = __ldg(reinterpret_cast<const int4*>(map.tmap + (tile * map.K + k_first + my_j) * (int64_t)kTileM) + lane);
-          ok = mbar_wait_all(smem_u32(&ctl->b_empty[b_slot]), b_phase ^ 1u, abort_flag, 36);
-          if (!ok) break;
-          const uint32_t bar = smem_u32(&ctl->b_full[b_slot]);
-          const uint32_t stage = b_ring + (uint32_t)b_slot * quad_bytes + (uint32_t)pw * (uint32_t)p.b_slot_bytes;
-          if (lane == 0) {
-            if (my_j >= 0) mbar_arrive_expect_tx(bar, (uint32_t)b_blocks * kABlockBytes); else mbar_arrive(bar);
-          }
-          __syncwarp();
-          if (my_j >= 0) {
-            for (int b = 0; b < b_blocks; ++b)
-              tma_gather4(stage + (uint32_t)b * kABlockBytes + (uint32_t)lane * 512u, gath_desc, bar, gath_col0 + b * per_line, idx.x,
-                          idx.y, idx.z, idx.w);
-          }
-          if (++b_slot == p.b_slots) {
-            b_slot = 0;
-            b_phase ^= 1u;
-          }
-        }
-      }
-    } else {
-    const int pw = warp - kFirstProducerWarp;
-    struct Cursor {
-      int64_t tile;
-      uint32_t m, m_next, b_count;
-      int a_slot, b_slot;
-      uint32_t a_phase, b_phase;
-      bool in_tile;
-    };
-    struct Task {
-      int kind;                 // 0 none, 1 dY tile, 2 X rows
-      int64_t tile;
-      int slot;
-      uint32_t parity;
-      int my_j;                 // kind 2: offset (within the group) this warp copies, or -1
-    };
-    auto cursor = [&]() {
-      Cursor c;
-      c.tile = tile_begin;
-      c.m = 0;
-      c.m_next = tile_begin < tile_end ? tile_mask(tile_begin) : 0u;
-      c.b_count = 0;
-      c.a_slot = c.b_slot = 0;
-      c.a_phase = c.b_phase = 0;
-      c.in_tile = false;
-      return c;
-    };
-    auto next = [&](Cursor& c) {
-      Task t{0, 0, 0, 0u, -1};
-      for (;;) {
-        if (c.tile >= tile_end) return t;
-        if (!c.in_tile) {
-          c.m = c.m_next;
-          c.m_next = c.tile + tile_step < tile_end ? tile_mask(c.tile + tile_step) : 0u;
-          if (!c.m) {
-            c.tile += tile_step;
-            continue;
-          }
-          c.in_tile = true;
-          t = Task{1, c.tile, c.a_slot, c.a_phase, -1};
-          if (++c.a_slot == p.a_slots) {
-            c.a_slot = 0;
-            c.a_phase ^= 1u;
-          }
-          return t;
-        }
-        // `quad` offsets per slot: warp q copies the q-th of them; with one offset per slot the warps take turns
-        int my_j = -1;
-        for (int q = 0; q < p.quad && c.m; ++q) {
-          const int j = __ffs(c.m) - 1;
-          c.m &= c.m - 1;
-          if ((p.quad == 1 ? (int)(c.b_count & (kProducerWarps - 1)) : q) == pw) my_j = j;
-        }
-        t = Task{2, c.tile, c.b_slot, c.b_phase, my_j};
-        ++c.b_count;
-        if (++c.b_slot == p.b_slots) {
-          c.b_slot = 0;
-          c.b_phase ^= 1u;
-        }
-        if (!c.m) {
-          c.in_tile = false;
-          c.tile += tile_step;
-        }
-        return t;
-      }
-    };
-    int a_mine = 0;                                   // column blocks of the dY tile this warp copies (block b: warp b % 4)
-    for (int b = pw; b < a_blocks; b += kProducerWarps) ++a_mine;
-    auto load_rows = [&](const Task& t) {
-      int4 rows = make_int4(-1, -1, -1, -1);
-      if (t.kind == 1 && a_mine) {
-        const int64_t pos = t.tile * kTileM + 4 * lane;
-        if (!p.order) {
-          rows = make_int4((int)pos, (int)pos + 1, (int)pos + 2, (int)pos + 3);
-        } else if (pos + 3 < p.n_rows && (reinterpret_cast<uintptr_t>(p.order) & 15) == 0) {
-          rows = __ldg(reinterpret_cast<const int4*>(p.order + pos));
-        } else {
-          // the last tile's line may run past the end of `order`: read only what exists
-          rows.x = pos + 0 < p.n_rows ? __ldg(p.order + pos + 0) : -1;
-          rows.y = pos + 1 < p.n_rows ? __ldg(p.order + pos + 1) : -1;
-          rows.z = pos + 2 < p.n_rows ? __ldg(p.order + pos + 2) : -1;
-          rows.w = pos + 3 < p.n_rows ? __ldg(p.order + pos + 3) : -1;
-        }
-        if (pos + 0 >= p.n_rows) rows.x = -1;
-        if (pos + 1 >= p.n_rows) rows.y = -1;
-        if (pos + 2 >= p.n_rows) rows.z = -1;
-        if (pos + 3 >= p.n_rows) rows.w = -1;
-      } else if (t.kind == 2 && t.my_j >= 0) {
-        rows = __ldg(reinterpret_cast<const int4*>(map.tmap + (t.tile * map.K + k_first + t.my_j) * (int64_t)kTileM) + lane);
-      }
-      return rows;
-    };
+  if (warp >= kWgradRowWarp0) {
+    // =============================================================== rows
+    // One sequence of items: per tile its tile operand (ring 1; every warp has 8 of its rows), then one item per offset
+    // (ring 2; four groups of four warps take them in turn, a warp has 32 rows), all column blocks of a row.  Since every
+    // warp waits for every slot of ring 1, none runs ahead by more than that ring; in ring 2 a warp's last item but one
+    // tells it which lap the consumer is in as long as the ring is no shorter than the number of groups, else it waits for
+    // every slot there too (a wait names a phase by its parity alone).
+    const int row_warp = warp - kWgradRowWarp0;
+    const int group = row_warp / kRowGroupWarps;
+    const int row0 = row_warp % kRowGroupWarps * 32, t_row0 = row_warp * (kTileM / (kRowGroups * kRowGroupWarps));
+    const bool every_slot = p.b_slots < kRowGroups;
+    const char* x = static_cast<const char*>(p.x) + (size_t)ci0 * ESIZE;
+    const char* dy = static_cast<const char*>(p.dy) + (size_t)co0 * ESIZE;
+    const int x_bytes = ci_cnt * ESIZE, dy_bytes = co_cnt * ESIZE, x_pitch = p.cin * ESIZE, dy_pitch = p.cout * ESIZE;
+    const char* t_src = p.swap ? x : dy;
+    const char* g_src = p.swap ? dy : x;
+    const int t_bytes = p.swap ? x_bytes : dy_bytes, g_bytes = p.swap ? dy_bytes : x_bytes;
+    const int t_pitch = p.swap ? x_pitch : dy_pitch, g_pitch = p.swap ? dy_pitch : x_pitch;
+    int a_slot = 0, b_slot = 0, turn = 0;
+    uint32_t a_phase = 0, b_phase = 0;
     bool ok = true;
-    auto issue = [&](const Task& t, const int4& rows) {
-      if (t.kind == 1) {
-        ok = mbar_wait_all(smem_u32(&ctl->a_empty[t.slot]), t.parity ^ 1u, abort_flag, 35);
-        if (!ok) return;
-        const uint32_t bar = smem_u32(&ctl->a_full[t.slot]);
-        const uint32_t slot_base = a_ring + (uint32_t)t.slot * (uint32_t)p.a_slot_bytes;
-        if (lane == 0) {
-          if (a_mine) mbar_arrive_expect_tx(bar, (uint32_t)a_mine * kABlockBytes); else mbar_arrive(bar);
-          if (p.dense_tiles)
-            for (int b = pw; b < a_blocks; b += kProducerWarps)
-              tma_load_2d(slot_base + (uint32_t)b * kABlockBytes, &tile_box_desc, bar, tile_col0 + b * per_line,
-                          (int)(t.tile * kTileM));
-        }
-        __syncwarp();
-        if (!p.dense_tiles)
-          for (int b = pw; b < a_blocks; b += kProducerWarps)
-            tma_gather4(slot_base + (uint32_t)b * kABlockBytes + (uint32_t)lane * 512u, tile_desc, bar, tile_col0 + b * per_line,
-                        rows.x, rows.y, rows.z, rows.w);
-      } else {
-        ok = mbar_wait_all(smem_u32(&ctl->b_empty[t.slot]), t.parity ^ 1u, abort_flag, 36);
-        if (!ok) return;
-        const uint32_t bar = smem_u32(&ctl->b_full[t.slot]);
-        const uint32_t stage = b_ring + (uint32_t)t.slot * quad_bytes + (uint32_t)(p.quad == 1 ? 0 : pw) * (uint32_t)p.b_slot_bytes;
-        if (lane == 0) {
-          if (t.my_j >= 0) mbar_arrive_expect_tx(bar, (uint32_t)b_blocks * kABlockBytes); else mbar_arrive(bar);
-        }
-        __syncwarp();
-        if (t.my_j >= 0) {
-          for (int b = 0; b < b_blocks; ++b)
-            tma_gather4(stage + (uint32_t)b * kABlockBytes + (uint32_t)lane * 512u, gath_desc, bar, gath_col0 + b * per_line, rows.x,
-                        rows.y, rows.z, rows.w);
-        }
-      }
+    uint32_t sent = 0;                                        // barrier of the item whose copies are under way, not yet announced
+    bool pend = false, pend_b = false;
+    int pend_slot = 0, pend_idx = -1;
+    uint32_t pend_parity = 0;
+    auto announce = [&]() {
+      __syncwarp();
+      if (sent && lane == 0) mbar_arrive(sent);
+      sent = 0;
     };
-    Cursor fetch = cursor();
-    Task queued[kAhead];
-    int4 queued_rows[kAhead];
-#pragma unroll
-    for (int d = 0; d < kAhead; ++d) {
-      queued[d] = next(fetch);
-      queued_rows[d] = load_rows(queued[d]);
-    }
-    while (queued[0].kind != 0 && ok) {
-      issue(queued[0], queued_rows[0]);
-#pragma unroll
-      for (int d = 0; d + 1 < kAhead; ++d) {
-        queued[d] = queued[d + 1];
-        queued_rows[d] = queued_rows[d + 1];
+    auto wait_for = [&](bool is_b, int slot, uint32_t parity) {
+      const uint32_t empty = smem_u32(is_b ? &ctl->b_empty[slot] : &ctl->a_empty[slot]);
+      if (__all_sync(0xFFFFFFFFu, mbar_try_now(empty, parity ^ 1u))) return true;
+      // the slot's release may depend on what this warp has not announced yet
+      cp_async_wait_all();
+      announce();
+      return mbar_wait_all(empty, parity ^ 1u, abort_flag, is_b ? 36 : 35);
+    };
+    auto run = [&]() {
+      ok = wait_for(pend_b, pend_slot, pend_parity);
+      if (!ok) return;
+      if (pend_b) {
+        const uint32_t dst = b_ring + (uint32_t)pend_slot * (uint32_t)p.b_slot_bytes;
+        for (int b = 0; b * 128 < g_bytes; ++b)
+          fetch_block<32, kBase32>(dst + (uint32_t)b * kABlockBytes, row0, pend_idx, g_src + b * 128, g_pitch, p.n_src,
+                                   min(128, g_bytes - b * 128), lane);
+      } else {
+        const uint32_t dst = a_ring + (uint32_t)pend_slot * (uint32_t)p.a_slot_bytes;
+        for (int b = 0; b * 128 < t_bytes; ++b)
+          fetch_block<8, kBase32>(dst + (uint32_t)b * kABlockBytes, t_row0, pend_idx, t_src + b * 128, t_pitch, p.n_rows,
+                                  min(128, t_bytes - b * 128), lane);
       }
-      queued[kAhead - 1] = next(fetch);
-      queued_rows[kAhead - 1] = load_rows(queued[kAhead - 1]);
-    }
-    }
+      cp_async_commit();
+      cp_async_wait_group<1>();                               // the item before this one has landed: announce it
+      announce();
+      sent = smem_u32(pend_b ? &ctl->b_full[pend_slot] : &ctl->a_full[pend_slot]);
+    };
+    auto queue = [&](bool is_b, int slot, uint32_t parity, int idx) {
+      if (pend) run();
+      pend = true;
+      pend_b = is_b;
+      pend_slot = slot;
+      pend_parity = parity;
+      pend_idx = idx;
+    };
+    walk_tiles(p, map, tile_begin, tile_step, word, shift, group_bits, lane, [&](int64_t tile, uint32_t m) {
+      const int64_t pos = tile * kTileM + t_row0 + (lane & 7);
+      queue(false, a_slot, a_phase, pos < p.n_rows ? (p.order ? __ldg(p.order + pos) : (int)pos) : -1);
+      if (++a_slot == p.a_slots) {
+        a_slot = 0;
+        a_phase ^= 1u;
+      }
+      while (m && ok) {
+        if (turn == group) {
+          const int j = __ffs(m) - 1;
+          queue(true, b_slot, b_phase, __ldg(map.tmap + (tile * map.K + k_first + j) * (int64_t)kTileM + row0 + lane));
+        } else if (every_slot) {
+          if (pend) run();
+          pend = false;
+          if (ok) ok = wait_for(true, b_slot, b_phase);
+        }
+        m &= m - 1;
+        turn = (turn + 1) & (kRowGroups - 1);
+        if (++b_slot == p.b_slots) {
+          b_slot = 0;
+          b_phase ^= 1u;
+        }
+      }
+      return ok;
+    });
+    if (pend && ok) run();
+    cp_async_wait_all();
+    announce();
   } else if (warp == kMmaWarp) {
-    // =============================================================== MMA issuer
-    if (lane == 0) {
-      int a_slot = 0, b_slot = 0;
-      uint32_t a_phase = 0, b_phase = 0;
-      uint32_t touched = 0;
-      bool ok = true;
-      const int rows_per_step = 32 / p.esize;                  // reduction rows per MMA (16 or 8)
-      const int ksteps = kTileM / rows_per_step;
-      const uint32_t step_bytes = (uint32_t)rows_per_step * 128u;
-      const uint32_t sbo = base32 ? 512u : 1024u, layout = base32 ? 1u : 2u;
-      const uint32_t idesc = p.idesc_base | ((uint32_t)(p.ci_blk >> 3) << 17);
-      const uint64_t desc_hi = smem_desc(0u, kABlockBytes, sbo, layout);
-      uint32_t m_next = tile_begin < tile_end ? tile_mask(tile_begin) : 0u;
-      for (int64_t tile = tile_begin; tile < tile_end && ok; tile += tile_step) {
-        uint32_t m = m_next;
-        if (tile + tile_step < tile_end) m_next = tile_mask(tile + tile_step);
-        if (!m) continue;
-        ok = mbar_wait(smem_u32(&ctl->a_full[a_slot]), a_phase, abort_flag, 37);
-        if (!ok) break;
-        const uint32_t a_lo = (a_ring + (uint32_t)a_slot * (uint32_t)p.a_slot_bytes) >> 4;
-        while (m && ok) {
-          ok = mbar_wait(smem_u32(&ctl->b_full[b_slot]), b_phase, abort_flag, 38);
-          if (!ok) break;
-          tc_fence_after();
-          for (int q = 0; q < p.quad && m; ++q) {
-            const int j = __ffs(m) - 1;
-            m &= m - 1;
-            const uint32_t b_lo = (b_ring + (uint32_t)b_slot * quad_bytes + (uint32_t)q * (uint32_t)p.b_slot_bytes) >> 4;
-            const uint32_t d_addr = tmem_base + (uint32_t)(j * p.ci_blk);
-            const uint32_t first = ((touched >> j) & 1u) ? 1u : 0u;
-            for (int ks = 0; ks < ksteps; ++ks) {
-              const uint64_t da = desc_hi | (uint64_t)((p.swap ? b_lo : a_lo) + ks * (step_bytes >> 4));   // dY rows (M)
-              const uint64_t db = desc_hi | (uint64_t)((p.swap ? a_lo : b_lo) + ks * (step_bytes >> 4));   // X rows (N)
-              if (p.esize == 2)
-                mma_f16(d_addr, da, db, idesc, ks == 0 ? first : 1u);
-              else
-                mma_tf32(d_addr, da, db, idesc, ks == 0 ? first : 1u);
-            }
-            touched |= 1u << j;
+    // =============================================================== MMA issuer (see planned_gather_kernel)
+    int a_slot = 0, b_slot = 0;
+    uint32_t a_phase = 0, b_phase = 0;
+    uint32_t touched = 0;
+    bool ok = true;
+    constexpr int kRowsPerStep = 32 / ESIZE;                   // reduction rows per MMA (16 or 8)
+    constexpr int kSteps = kTileM / kRowsPerStep;
+    constexpr uint32_t kStep16 = kRowsPerStep * 128 / 16;
+    const uint32_t idesc = p.idesc_base | ((uint32_t)(p.ci_blk >> 3) << 17);
+    const uint64_t desc_hi = smem_desc(0u, kABlockBytes, kBase32 ? 512u : 1024u, kBase32 ? 1u : 2u);
+    walk_tiles(p, map, tile_begin, tile_step, word, shift, group_bits, lane, [&](int64_t, uint32_t m) {
+      ok = mbar_wait_all(smem_u32(&ctl->a_full[a_slot]), a_phase, abort_flag, 37);
+      if (!ok) return false;
+      const uint32_t t_lo = (a_ring + (uint32_t)a_slot * (uint32_t)p.a_slot_bytes) >> 4;
+      while (m) {
+        const int j = __ffs(m) - 1;
+        m &= m - 1;
+        ok = mbar_wait_all(smem_u32(&ctl->b_full[b_slot]), b_phase, abort_flag, 38);
+        if (!ok) return false;
+        fence_proxy_async();                                   // rows were written by cp.async
+        tc_fence_after();
+        const uint32_t g_lo = (b_ring + (uint32_t)b_slot * (uint32_t)p.b_slot_bytes) >> 4;
+        const uint32_t a_lo = p.swap ? g_lo : t_lo, b_lo = p.swap ? t_lo : g_lo;   // dY rows (M), X rows (N)
+        const uint32_t d_addr = tmem_base + (uint32_t)(j * p.ci_blk);
+        const uint32_t add = (touched >> j) & 1u;
+        if (elect_one()) {
+#pragma unroll
+          for (int ks = 0; ks < kSteps; ++ks) {
+            const uint64_t da = desc_hi | (uint64_t)(a_lo + ks * kStep16);
+            const uint64_t db = desc_hi | (uint64_t)(b_lo + ks * kStep16);
+            if (ESIZE == 2)
+              mma_f16(d_addr, da, db, idesc, ks == 0 ? add : 1u);
+            else
+              mma_tf32(d_addr, da, db, idesc, ks == 0 ? add : 1u);
           }
           mma_commit(smem_u32(&ctl->b_empty[b_slot]));
-          if (++b_slot == p.b_slots) {
-            b_slot = 0;
-            b_phase ^= 1u;
-          }
         }
-        mma_commit(smem_u32(&ctl->a_empty[a_slot]));
-        if (++a_slot == p.a_slots) {
-          a_slot = 0;
-          a_phase ^= 1u;
+        touched |= 1u << j;
+        if (++b_slot == p.b_slots) {
+          b_slot = 0;
+          b_phase ^= 1u;
         }
       }
-      if (ok) {
-        ctl->touched = touched;
-        mma_commit(smem_u32(&ctl->acc_full));
-        mbar_arrive(smem_u32(&ctl->acc_full));
+      if (elect_one()) mma_commit(smem_u32(&ctl->a_empty[a_slot]));
+      if (++a_slot == p.a_slots) {
+        a_slot = 0;
+        a_phase ^= 1u;
       }
+      return true;
+    });
+    if (ok && elect_one()) {
+      ctl->touched = touched;
+      mma_commit(smem_u32(&ctl->acc_full));
+      mbar_arrive(smem_u32(&ctl->acc_full));
     }
     __syncwarp();
   } else {
@@ -795,16 +694,18 @@ __global__ void __launch_bounds__(kThreads, 1) planned_wgrad_kernel(const WgradP
       tc_fence_after();
       const uint32_t touched = ctl->touched;
       const int co = warp * 32 + lane;                           // accumulator row = output channel
+      const int co_w = min(p.cout, 128);
+      float* mine = p.partial + (size_t)blockIdx.x * p.group * p.ci_blk * co_w + co;
       for (int j = 0; j < g_count; ++j) {
-        float* dst = p.partial + (((size_t)chunk * p.K + (k_first + j)) * p.cin + ci0) * p.cout + co0 + co;
         const bool live = (touched >> j) & 1u;
         for (int c0 = 0; c0 < ci_cnt; c0 += 16) {
           uint32_t v[32];
           tmem_ld16(tmem_base + ((uint32_t)(warp * 32) << 16) + (uint32_t)(j * p.ci_blk + c0), v);
           tmem_ld_wait();
+          float* dst = mine + (size_t)(j * p.ci_blk + c0) * co_w;
           if (co < co_cnt) {
 #pragma unroll
-            for (int c = 0; c < 16; ++c) dst[(size_t)(c0 + c) * p.cout] = live ? __uint_as_float(v[c]) : 0.f;
+            for (int c = 0; c < 16; ++c) dst[(size_t)c * co_w] = live ? __uint_as_float(v[c]) : 0.f;
           }
         }
       }
@@ -820,6 +721,60 @@ __global__ void __launch_bounds__(kThreads, 1) planned_wgrad_kernel(const WgradP
   if (warp == kMmaWarp) {
     tc_fence_after();
     tmem_dealloc(tmem_base, (uint32_t)p.tmem_cols);
+  }
+}
+
+template <typename T> __device__ __forceinline__ T from_f(float v);
+template <> __device__ __forceinline__ float from_f<float>(float v) { return v; }
+template <> __device__ __forceinline__ __half from_f<__half>(float v) { return __float2half_rn(v); }
+template <> __device__ __forceinline__ __nv_bfloat16 from_f<__nv_bfloat16>(float v) { return __float2bfloat16_rn(v); }
+
+// dW[k][ci][co] = sum over the CTAs of its combination, in order: eight slices of the CTAs per block, added from shared
+// memory.  A block takes 32 x 4 consecutive output channels' worth of one (k, ci) row or several.
+template <typename T>
+__global__ void __launch_bounds__(256) wgrad_sum_kernel(const WgradParams p, T* __restrict__ dw) {
+  __shared__ float4 part[8][32];
+  const int slice = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int quads = p.cout >> 2;                                 // cout is a multiple of 8
+  const int64_t n = (int64_t)p.K * p.cin * quads, i = (int64_t)blockIdx.x * 32 + lane;
+  float4 sum = make_float4(0.f, 0.f, 0.f, 0.f);
+  int k = 0, ci = 0, co = 0;
+  if (i < n) {
+    co = (int)(i % quads) * 4;
+    ci = (int)(i / quads % p.cin);
+    k = (int)(i / quads / p.cin);
+    const int kgroup = k / p.group, j = k - kgroup * p.group;
+    const int coblk = co / 128, ciblk = ci / p.ci_blk;
+    const int combo = (kgroup * p.n_coblk + coblk) * p.n_ciblk + ciblk;
+    const int co_w = min(p.cout, 128);
+    const size_t cta_floats = (size_t)p.group * p.ci_blk * co_w;
+    const float* src = p.partial + ((size_t)j * p.ci_blk + (ci - ciblk * p.ci_blk)) * co_w + (co - coblk * 128);
+    const int first = p.cta_table[combo], end = p.cta_table[combo + 1];
+#pragma unroll 4
+    for (int c = first + slice; c < end; c += 8) {
+      const float4 v = *reinterpret_cast<const float4*>(src + c * cta_floats);
+      sum.x += v.x;
+      sum.y += v.y;
+      sum.z += v.z;
+      sum.w += v.w;
+    }
+  }
+  part[slice][lane] = sum;
+  __syncthreads();
+  if (slice == 0 && i < n) {
+#pragma unroll
+    for (int s = 1; s < 8; ++s) {
+      const float4 v = part[s][lane];
+      sum.x += v.x;
+      sum.y += v.y;
+      sum.z += v.z;
+      sum.w += v.w;
+    }
+    T* out = dw + ((size_t)k * p.cin + ci) * p.cout + co;
+    out[0] = from_f<T>(sum.x);
+    out[1] = from_f<T>(sum.y);
+    out[2] = from_f<T>(sum.z);
+    out[3] = from_f<T>(sum.w);
   }
 }
 
