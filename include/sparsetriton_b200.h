@@ -91,6 +91,9 @@ int st_set_dense_tiles(int enable);
  * Replaces the two torch.full(-1) fills of HashTable.__init__, sparsetriton/utils/hash.py:428-429. */
 int st_hash_clear(int64_t* keys, int32_t* vals, int64_t capacity, void* stream);
 
+/* st_hash_clear, and n_zero (<= 32) further words set to zero by the same launch. */
+int st_hash_clear_words(int64_t* keys, int32_t* vals, int64_t capacity, int32_t* zero, int n_zero, void* stream);
+
 /* Insert n coordinates; value = row index; a repeated coordinate keeps its largest row.
  * Replaces HashTable.insert -> build_hash_table_kernel, sparsetriton/utils/hash.py:516-544, 193-258.
  * status: device int32, ST_DEV_TABLE_FULL is OR-ed in if some key found no slot, ST_DEV_BAD_INDEX if a
@@ -244,6 +247,12 @@ int st_conv_dgrad_planned(int dtype, const void* dY, const void* W, const int32_
 int st_conv_wgrad_planned(int dtype, const void* X, const void* dY, const int32_t* nbr, const int32_t* row_order,
                           const int32_t* tmap, const uint32_t* tmask, void* dW, int64_t n_in, int64_t n_out, int K,
                           int cin, int cout, void* workspace, int64_t workspace_bytes, void* stream);
+
+/* st_conv_wgrad_planned with dW in fp32 whatever the feature dtype (the fp32 sums as they are: what fp32 master weights
+ * take).  ST_ERR_UNSUPPORTED for 16-bit features on shapes the tensor-core kernels do not serve. */
+int st_conv_wgrad_planned_f32(int dtype, const void* X, const void* dY, const int32_t* nbr, const int32_t* row_order,
+                              const int32_t* tmap, const uint32_t* tmask, float* dW, int64_t n_in, int64_t n_out, int K, int cin,
+                              int cout, void* workspace, int64_t workspace_bytes, void* stream);
 
 /* st_conv_wgrad_planned over a copy of dY in the plan's row order, made by a call of its own (on another stream, say).
  * st_conv_wgrad_planned itself makes no copy and is as fast.
@@ -408,6 +417,27 @@ int st_bn_forward_stats(int dtype, const void* X, const int32_t* batch, const in
 int st_bn_backward(int dtype, const void* X, const void* dY, const int32_t* batch, int64_t n, int C, int B, const float* mean,
                    const float* rstd, const float* weight, const float* bias, int relu, int batch_stats,
                    const float* inv_count, float* sums, void* dX, float* dW, float* dB, int32_t* status, void* stream);
+
+/* Y = the affine part over running statistics: (X - mean[c]) / sqrt(var[c] + eps) * weight[c] + bias[c], relu optionally; one
+ * launch where the rows allow the streaming kernel.  rstd_scratch: C floats.  st_bn_rstd: 1 / sqrt(var + eps) alone. */
+int st_bn_apply_running(int dtype, const void* X, int64_t n, int C, const float* mean, const float* var, float eps,
+                        const float* weight, const float* bias, int relu, float* rstd_scratch, void* Y, void* stream);
+int st_bn_rstd(const float* var, int C, float eps, float* rstd, void* stream);
+
+/* What the normalisation layers derive from the batch column of a coordinate set: ids[i] (n int32), 1 / max(rows, 1) and the
+ * first row (-1: none) of each of B samples; rows outside [0, B) join none.  counts: B + 2 uint32, scratch; the last one is zero afterwards (a
+ * status word for the layers). */
+int st_bn_batch_info(const void* coords, int64_t n, int coord_dtype, int B, int32_t* ids, uint32_t* counts, int32_t* first_row,
+                     float* inv_count, void* stream);
+
+/* ---------------------------------------------------------------- results for a polling host --- */
+
+/* Writes up to eight device words, and with kernel_status the four status words behind them, into host16 (16 int32 of pinned
+ * host memory), then host16[15] <- ticket: a host that polls for its ticket needs no event and no copy. */
+int st_publish(const int32_t* words, int n_words, int kernel_status, int32_t* host16, int32_t ticket, void* stream);
+/* The same for the largest value of each coordinate column (host16[0..3]).  scratch: five uint32, zero, zero again after. */
+int st_coord_extent(const void* coords, int64_t n, int coord_dtype, uint32_t* scratch, int32_t* host16, int32_t ticket,
+                    void* stream);
 
 /* Hash-on-the-fly forms: no stored map; every tile recomputes
  *   curr = out*lookup_stride - off[k], bounds-checks it against lookup_shape and probes the table.

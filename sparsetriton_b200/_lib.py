@@ -12,6 +12,7 @@ import torch
 
 _PKG = os.path.dirname(os.path.abspath(__file__))
 LIB_PATH = os.path.join(_PKG, "_native", "libsparsetriton_b200.so")
+HOST_PATH = os.path.join(_PKG, "_native", "_st_host.so")
 
 ST_I16, ST_I32 = 0, 1
 ST_F32, ST_F16, ST_BF16 = 0, 1, 2
@@ -38,6 +39,10 @@ _SIGNATURES = {
     "st_set_tensor_cores": ([_INT], _INT),
     "st_set_tma": ([_INT], _INT),
     "st_hash_clear": ([_PTR, _PTR, _I64, _PTR], _INT),
+    "st_hash_clear_words": ([_PTR, _PTR, _I64, _PTR, _INT, _PTR], _INT),
+    "st_publish": ([_PTR, _INT, _INT, _PTR, _INT, _PTR], _INT),
+    "st_coord_extent": ([_PTR, _I64, _INT, _PTR, _PTR, _INT, _PTR], _INT),
+    "st_bn_batch_info": ([_PTR, _I64, _INT, _INT, _PTR, _PTR, _PTR, _PTR, _PTR], _INT),
     "st_hash_build": ([_PTR, _I64, _INT, _PTR, _PTR, _I64, _PTR, _PTR], _INT),
     "st_hash_query": ([_PTR, _I64, _INT, _PTR, _PTR, _I64, _PTR, _PTR], _INT),
     "st_outcoords_workspace_bytes": ([_I64, _INT, _INT, _INT], _I64),
@@ -58,7 +63,8 @@ _SIGNATURES = {
     "st_conv_wgrad": ([_INT, _PTR, _PTR, _PTR, _PTR, _I64, _I64, _INT, _INT, _INT, _PTR, _I64, _PTR], _INT),
 }
 _PLANNED_SIG = ([_INT, _PTR, _PTR, _PTR, _PTR, _PTR, _PTR, _PTR, _I64, _I64, _INT, _INT, _INT, _PTR, _I64, _PTR], _INT)
-for _n in ("st_conv_fwd_planned", "st_conv_dgrad_planned", "st_conv_wgrad_planned", "st_conv_wgrad_planned_presorted"):
+for _n in ("st_conv_fwd_planned", "st_conv_dgrad_planned", "st_conv_wgrad_planned", "st_conv_wgrad_planned_presorted",
+           "st_conv_wgrad_planned_f32"):
     _SIGNATURES[_n] = _PLANNED_SIG
 _SIGNATURES["st_conv_wgrad_presort"] = ([_INT, _PTR, _PTR, _I64, _INT, _INT, _INT, _PTR, _I64, _PTR], _INT)
 _SIGNATURES["st_map_plan_workspace_bytes"] = ([_I64, _INT], _I64)
@@ -74,6 +80,8 @@ _SIGNATURES["st_bn_backward_sums"] = ([_INT, _PTR, _PTR, _PTR, _I64, _INT, _INT,
 _SIGNATURES["st_bn_backward_apply"] = ([_INT, _PTR, _PTR, _PTR, _I64, _INT, _INT, _PTR, _PTR, _PTR, _PTR, _INT, _PTR, _PTR,
                                         _PTR, _PTR, _PTR], _INT)
 _F32 = ctypes.c_float
+_SIGNATURES["st_bn_rstd"] = ([_PTR, _INT, _F32, _PTR, _PTR], _INT)
+_SIGNATURES["st_bn_apply_running"] = ([_INT, _PTR, _I64, _INT, _PTR, _PTR, _F32, _PTR, _PTR, _INT, _PTR, _PTR, _PTR], _INT)
 _SIGNATURES["st_conv_wgrad_inverse_workspace_bytes"] = ([_INT, _I64, _INT, _INT, _INT], _I64)
 _SIGNATURES["st_conv_wgrad_inverse_planned"] = ([_INT, _PTR, _PTR, _PTR, _PTR, _PTR, _PTR, _I64, _I64, _INT, _INT, _INT, _PTR, _I64,
                                                  _PTR], _INT)
@@ -117,6 +125,24 @@ def lib():
             fn.restype = restype
         _lib = handle
     return _lib
+
+
+_host = None
+
+
+def host():
+    """The native host side (allocation, plans, autograd nodes: `sparsetriton_b200/host/`), loaded on first use."""
+    global _host
+    if _host is None:
+        lib()
+        if not os.path.exists(HOST_PATH):
+            raise RuntimeError(f"{HOST_PATH} is missing: build it with `python -m sparsetriton_b200.build`")
+        import importlib.util
+        spec = importlib.util.spec_from_file_location("_st_host", HOST_PATH)
+        module = importlib.util.module_from_spec(spec)
+        spec.loader.exec_module(module)
+        _host = module
+    return _host
 
 
 def check(rc, what):

@@ -249,8 +249,8 @@ int st_conv_dgrad_mirrored(int dtype, const void* dY, const void* W, const int32
 }
 
 static int wgrad_planned(int dtype, const void* X, const void* dY, const int32_t* nbr, const int32_t* row_order,
-                         const int32_t* tmap, const uint32_t* tmask, void* dW, int64_t n_in, int64_t n_out, int K, int cin,
-                         int cout, void* workspace, int64_t workspace_bytes, void* stream, bool presorted) {
+                         const int32_t* tmap, const uint32_t* tmask, int dw_dtype, void* dW, int64_t n_in, int64_t n_out, int K,
+                         int cin, int cout, void* workspace, int64_t workspace_bytes, void* stream, bool presorted) {
   int rc = check_conv_args("st_conv_wgrad", dtype, n_in, n_out, K, cin, cout);
   if (rc != ST_OK) return rc;
   if (!dW || (n_out > 0 && (!X || !dY || !nbr))) {
@@ -267,10 +267,11 @@ static int wgrad_planned(int dtype, const void* X, const void* dY, const int32_t
     int chunks = 0;
     const void* rows = presorted ? static_cast<char*>(workspace) + wgrad_sorted_offset(dtype, n_out, K, cin, cout) : dY;
     rc = tc_conv_wgrad(dtype, X, rows, nbr, MapPlan{presorted ? nullptr : row_order, tmap, tmask}, static_cast<float*>(workspace),
-                       &chunks, n_out, n_in, K, cin, cout, s, dW);
+                       &chunks, n_out, n_in, K, cin, cout, s, dw_dtype, dW);
     if (rc != ST_OK || chunks == 0) return rc;
-    return reduce_partials(dtype, static_cast<const float*>(workspace), chunks, (int64_t)K * cin * cout, dW, s);
+    return reduce_partials(dw_dtype, static_cast<const float*>(workspace), chunks, (int64_t)K * cin * cout, dW, s);
   }
+  if (dw_dtype != dtype) return ST_ERR_UNSUPPORTED;         // the CUDA-core kernels write the feature dtype
   StoredMap map{nbr, K};
   return by_dtype(dtype, [&](auto* tag) {
     using T = std::remove_pointer_t<decltype(tag)>;
@@ -282,8 +283,15 @@ static int wgrad_planned(int dtype, const void* X, const void* dY, const int32_t
 int st_conv_wgrad_planned(int dtype, const void* X, const void* dY, const int32_t* nbr, const int32_t* row_order,
                           const int32_t* tmap, const uint32_t* tmask, void* dW, int64_t n_in, int64_t n_out, int K, int cin,
                           int cout, void* workspace, int64_t workspace_bytes, void* stream) {
-  return wgrad_planned(dtype, X, dY, nbr, row_order, tmap, tmask, dW, n_in, n_out, K, cin, cout, workspace, workspace_bytes,
+  return wgrad_planned(dtype, X, dY, nbr, row_order, tmap, tmask, dtype, dW, n_in, n_out, K, cin, cout, workspace, workspace_bytes,
                        stream, /*presorted=*/false);
+}
+
+int st_conv_wgrad_planned_f32(int dtype, const void* X, const void* dY, const int32_t* nbr, const int32_t* row_order,
+                              const int32_t* tmap, const uint32_t* tmask, float* dW, int64_t n_in, int64_t n_out, int K, int cin,
+                              int cout, void* workspace, int64_t workspace_bytes, void* stream) {
+  return wgrad_planned(dtype, X, dY, nbr, row_order, tmap, tmask, ST_F32, dW, n_in, n_out, K, cin, cout, workspace,
+                       workspace_bytes, stream, /*presorted=*/false);
 }
 
 int st_conv_wgrad_presort(int dtype, const void* dY, const int32_t* row_order, int64_t n_out, int K, int cin, int cout,
@@ -305,7 +313,7 @@ int st_conv_wgrad_presort(int dtype, const void* dY, const int32_t* row_order, i
 int st_conv_wgrad_planned_presorted(int dtype, const void* X, const void* dY, const int32_t* nbr, const int32_t* row_order,
                                     const int32_t* tmap, const uint32_t* tmask, void* dW, int64_t n_in, int64_t n_out,
                                     int K, int cin, int cout, void* workspace, int64_t workspace_bytes, void* stream) {
-  return wgrad_planned(dtype, X, dY, nbr, row_order, tmap, tmask, dW, n_in, n_out, K, cin, cout, workspace, workspace_bytes,
+  return wgrad_planned(dtype, X, dY, nbr, row_order, tmap, tmask, dtype, dW, n_in, n_out, K, cin, cout, workspace, workspace_bytes,
                        stream, /*presorted=*/true);
 }
 
@@ -335,7 +343,7 @@ int st_conv_wgrad_inverse_planned(int dtype, const void* X, const void* dY, cons
   cudaStream_t s = (cudaStream_t)stream;
   int chunks = 0;
   return tc_conv_wgrad(dtype, X, dY, nullptr, MapPlan{row_order, tmap, tmask}, static_cast<float*>(workspace), &chunks, n_in,
-                       n_out, K, cin, cout, s, dW, true);
+                       n_out, K, cin, cout, s, dtype, dW, true);
 }
 
 int st_conv_wgrad(int dtype, const void* X, const void* dY, const int32_t* nbr, void* dW, int64_t n_in, int64_t n_out,

@@ -1619,8 +1619,8 @@ static bool prepare_wgrad(WgradPlan* plan, int dtype, const void* x, const void*
 }
 
 int tc_conv_wgrad(int dtype, const void* x, const void* dy, const int32_t* map, const MapPlan& rows, float* partial,
-                  int* n_chunks_out, int64_t n_rows, int64_t n_src, int K, int cin, int cout, cudaStream_t stream, void* dw,
-                  bool inverse_plan) {
+                  int* n_chunks_out, int64_t n_rows, int64_t n_src, int K, int cin, int cout, cudaStream_t stream, int dw_dtype,
+                  void* dw, bool inverse_plan) {
   WgradPlan plan;
   const bool has_plan = rows.tmap && rows.tmask;
   if (has_plan && g_tma_enabled && aligned16(x) && aligned16(dy) && n_src > 0 && n_src <= 0x7FFFFFFFll &&
@@ -1631,7 +1631,7 @@ int tc_conv_wgrad(int dtype, const void* x, const void* dy, const int32_t* map, 
     plan.p.partial = partial;
     plan.p.n_src = n_src;
     *n_chunks_out = 0;
-    return launch_wgrad_planned(plan, tc::PlannedRows{rows.tmap, rows.tmask, K, (K + 31) / 32}, dtype, dw, stream);
+    return launch_wgrad_planned(plan, tc::PlannedRows{rows.tmap, rows.tmask, K, (K + 31) / 32}, dw_dtype, dw, stream);
   }
   if (inverse_plan) {
     set_error("tc wgrad over the inverse plan needs a tile plan and 16-byte aligned tensors (st_set_tma(1))");
@@ -1676,6 +1676,23 @@ int tc_conv_wgrad_hashfly(int dtype, const void* x, const void* dy, const HashFl
 int tc_read_prof(long long* host_out, int n) {
   cudaDeviceSynchronize();
   return cudaMemcpyFromSymbol(host_out, tc::g_prof, sizeof(long long) * n) == cudaSuccess ? ST_OK : ST_ERR_CUDA;
+}
+
+// Device address of the status words on the current device.
+int tc_status_address(int32_t** out) {
+  static int32_t* known[kMaxDevices] = {};
+  int32_t*& p = known[current_device()];
+  if (!p) {
+    void* addr = nullptr;
+    const cudaError_t e = cudaGetSymbolAddress(&addr, tc::g_status);
+    if (e != cudaSuccess) {
+      set_error("tc_status_address: %s", cudaGetErrorString(e));
+      return ST_ERR_CUDA;
+    }
+    p = static_cast<int32_t*>(addr);
+  }
+  *out = p;
+  return ST_OK;
 }
 
 int tc_read_status(int32_t* host_out4, cudaStream_t stream, bool wait) {

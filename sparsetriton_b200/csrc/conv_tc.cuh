@@ -59,12 +59,12 @@ int tc_conv_wgrad_hashfly(int dtype, const void* x, const void* dy, const HashFl
 // Tensor-core weight gradient: fills fp32 partials (n_chunks, K, cin, cout) that the caller reduces.
 bool tc_wgrad_supported(int dtype, int64_t n_rows, int K, int cin, int cout);
 int64_t tc_wgrad_partial_bytes(int dtype, int64_t n_rows, int K, int cin, int cout);
-// Over a tile plan the whole weight gradient is made, into dw, and *n_chunks_out is 0 (nothing is left to reduce).
+// Over a tile plan the whole weight gradient is made, into dw (of type dw_dtype), and *n_chunks_out is 0 (nothing is left to reduce).
 // inverse_plan: `plan` is the tile plan of the INVERSE map; then n_rows counts the rows of x (the plan's rows) and
 // n_src the rows of dy (the rows the plan's entries name).
 int tc_conv_wgrad(int dtype, const void* x, const void* dy, const int32_t* map, const MapPlan& plan, float* partial,
-                  int* n_chunks_out, int64_t n_rows, int64_t n_src, int K, int cin, int cout, cudaStream_t stream, void* dw,
-                  bool inverse_plan = false);
+                  int* n_chunks_out, int64_t n_rows, int64_t n_src, int K, int cin, int cout, cudaStream_t stream, int dw_dtype,
+                  void* dw, bool inverse_plan = false);
 int64_t tc_wgrad_planned_bytes(int dtype, int64_t n_rows, int K, int cin, int cout);
 // Whether a copy of dY in tile order is offered for this layer (st_conv_wgrad_presort), and that copy alone; with it made
 // beforehand, tc_conv_wgrad takes the copy as dy and no order.

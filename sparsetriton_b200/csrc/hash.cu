@@ -11,7 +11,8 @@ namespace st {
 constexpr int kThreads = 256;
 
 __global__ void __launch_bounds__(kThreads)
-hash_clear_kernel(unsigned long long* keys, int32_t* vals, int64_t capacity) {
+hash_clear_kernel(unsigned long long* keys, int32_t* vals, int64_t capacity, int32_t* zero, int n_zero) {
+  if (blockIdx.x == 0 && threadIdx.x < n_zero) zero[threadIdx.x] = 0;
   // two slots per thread so that key stores are 16 bytes wide
   int64_t i = ((int64_t)blockIdx.x * kThreads + threadIdx.x) * 2;
   if (i + 1 < capacity && (reinterpret_cast<uintptr_t>(keys) & 15) == 0) {
@@ -129,14 +130,18 @@ using namespace st;
 extern "C" {
 
 int st_hash_clear(int64_t* keys, int32_t* vals, int64_t capacity, void* stream) {
-  if (capacity < 0 || (capacity > 0 && (!keys || !vals))) {
+  return st_hash_clear_words(keys, vals, capacity, nullptr, 0, stream);
+}
+
+int st_hash_clear_words(int64_t* keys, int32_t* vals, int64_t capacity, int32_t* zero, int n_zero, void* stream) {
+  if (capacity < 0 || (capacity > 0 && (!keys || !vals)) || n_zero < 0 || n_zero > 32 || (n_zero > 0 && !zero)) {
     set_error("st_hash_clear: bad arguments");
     return ST_ERR_ARG;
   }
-  if (capacity == 0) return ST_OK;
-  int64_t threads = (capacity + 1) / 2;
+  if (capacity == 0 && n_zero == 0) return ST_OK;
+  int64_t threads = capacity > 0 ? (capacity + 1) / 2 : 1;
   { hash_clear_kernel<<<(unsigned)((threads + kThreads - 1) / kThreads), kThreads, 0, (cudaStream_t)stream>>>(
-      reinterpret_cast<unsigned long long*>(keys), vals, capacity); note_launches(1); }
+      reinterpret_cast<unsigned long long*>(keys), vals, capacity, zero, n_zero); note_launches(1); }
   return check_launch("st_hash_clear");
 }
 

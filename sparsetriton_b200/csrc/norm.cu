@@ -506,7 +506,8 @@ __global__ void __launch_bounds__(stream::kThreads, 2)
                      int B, const float* __restrict__ p0 /* MODE 0: unused, else mean */, const float* __restrict__ rstd,
                      const float* __restrict__ w, const float* __restrict__ bias, int relu,
                      const float* __restrict__ sums_in, const float* __restrict__ inv_count, float* __restrict__ sums_out,
-                     T* __restrict__ out, const int32_t* __restrict__ first_row, int64_t chunks_per_block, int32_t* status) {
+                     T* __restrict__ out, const int32_t* __restrict__ first_row, int64_t chunks_per_block, int32_t* status,
+                     float var_eps /* MODE 2: >= 0: `rstd` holds variances, 1 / sqrt(v + var_eps) is meant */) {
   using namespace stream;
   constexpr int V = Vec<T>::V;
   constexpr int A = Ring<MODE>::kOperands, S = Ring<MODE>::kStages;
@@ -595,9 +596,8 @@ __global__ void __launch_bounds__(stream::kThreads, 2)
       const uint32_t parity = (uint32_t)(i / S) & 1u;
       const int64_t row_start = k * R;
       const int rows = (int)min((int64_t)R, n - row_start);
-      int ok = 1;
-      if (lane == 0) ok = mbar_wait(smem_u32(&full[s]), parity, abort_flag, status) ? 1 : 0;
-      if (!__shfl_sync(0xFFFFFFFFu, ok, 0)) break;
+      // every lane polls: a warp whose first lane alone waits goes on in fragments
+      if (!__all_sync(0xFFFFFFFFu, mbar_wait(smem_u32(&full[s]), parity, abort_flag, status))) break;
       const unsigned char* stage = ring_ptr + (size_t)s * Ring<MODE>::kStageBytes;
       const uint4* sx = reinterpret_cast<const uint4*>(stage);
       const uint4* sd = reinterpret_cast<const uint4*>(stage + (A - 1) * kChunkBytes);
@@ -647,6 +647,7 @@ __global__ void __launch_bounds__(stream::kThreads, 2)
             } else {
               a[i] = __ldg(p0 + sc + i);
               b[i] = __ldg(rstd + sc + i);
+              if (MODE == 2 && var_eps >= 0.f) b[i] = rsqrtf(b[i] + var_eps);
             }
             if (MODE == 3) {
               q0[i] = __ldg(sums_in + (sc + i) * 2);
@@ -850,11 +851,16 @@ int bn_sm_count() {
   return count[dev];
 }
 
+__global__ void __launch_bounds__(128) bn_rstd_kernel(const float* __restrict__ var, int C, float eps, float* __restrict__ rstd) {
+  const int c = blockIdx.x * 128 + threadIdx.x;
+  if (c < C) rstd[c] = rsqrtf(var[c] + eps);
+}
+
 // Launches bn_stream_kernel<T, MODE> over all n rows: two blocks per SM, each a contiguous range of chunks.
 template <typename T, int MODE>
 bool launch_stream(const T* x, const T* dy, const int32_t* batch, int64_t n, int C, int B, const float* p0, const float* rstd,
                    const float* w, const float* bias, int relu, const float* sums_in, const float* inv_count, float* sums_out,
-                   T* out, const int32_t* first_row, int32_t* status, cudaStream_t s) {
+                   T* out, const int32_t* first_row, int32_t* status, cudaStream_t s, float var_eps = -1.f) {
   auto kernel = bn_stream_kernel<T, MODE>;
   constexpr int smem = stream::Ring<MODE>::kBytes;
   static bool configured[kBnMaxDevices] = {};
@@ -873,7 +879,7 @@ bool launch_stream(const T* x, const T* dy, const int32_t* batch, int64_t n, int
   const int64_t per_block = (n_chunks + grid - 1) / grid;
   grid = (n_chunks + per_block - 1) / per_block;
   kernel<<<(unsigned)grid, stream::kThreads, smem, s>>>(x, dy, batch, n, C, B, p0, rstd, w, bias, relu, sums_in, inv_count,
-                                                         sums_out, out, first_row, per_block, status);
+                                                         sums_out, out, first_row, per_block, status, var_eps);
   return true;
 }
 
@@ -968,6 +974,40 @@ int st_bn_apply(int dtype, const void* X, const int32_t* batch, int64_t n, int C
   });
   note_launches(1);
   return check_launch("st_bn_apply");
+}
+
+int st_bn_rstd(const float* var, int C, float eps, float* rstd, void* stream) {
+  if (C < 1 || !var || !rstd) {
+    set_error("st_bn_rstd: bad arguments");
+    return ST_ERR_ARG;
+  }
+  bn_rstd_kernel<<<(unsigned)((C + 127) / 128), 128, 0, (cudaStream_t)stream>>>(var, C, eps, rstd);
+  note_launches(1);
+  return check_launch("st_bn_rstd");
+}
+
+int st_bn_apply_running(int dtype, const void* X, int64_t n, int C, const float* mean, const float* var, float eps,
+                        const float* weight, const float* bias, int relu, float* rstd_scratch, void* Y, void* stream) {
+  int rc = check_bn("st_bn_apply_running", dtype, n, C, 1);
+  if (rc != ST_OK) return rc;
+  if (n == 0) return ST_OK;
+  if (!X || !Y || !mean || !var || !rstd_scratch || !(eps >= 0.f)) {
+    set_error("st_bn_apply_running: bad arguments");
+    return ST_ERR_ARG;
+  }
+  bool done = false;
+  ST_BN_DISPATCH(dtype, {
+    done = stream_ok<T>(C, X, Y, nullptr) &&
+           launch_stream<T, 2>(static_cast<const T*>(X), nullptr, nullptr, n, C, 1, mean, var, weight, bias, relu, nullptr, nullptr,
+                               nullptr, static_cast<T*>(Y), nullptr, nullptr, (cudaStream_t)stream, eps);
+  });
+  if (done) {
+    note_launches(1);
+    return check_launch("st_bn_apply_running");
+  }
+  rc = st_bn_rstd(var, C, eps, rstd_scratch, stream);
+  if (rc != ST_OK) return rc;
+  return st_bn_apply(dtype, X, nullptr, n, C, 1, mean, rstd_scratch, weight, bias, relu, Y, nullptr, stream);
 }
 
 int st_bn_backward_sums(int dtype, const void* X, const void* dY, const int32_t* batch, int64_t n, int C, int B,

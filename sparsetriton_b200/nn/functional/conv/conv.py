@@ -8,14 +8,14 @@ from typing import Tuple, Union
 
 import torch
 
-from sparsetriton_b200 import _lib, trace
+from sparsetriton_b200 import _lib
 from sparsetriton_b200.config import ConvAlgo, get_conv_algo, get_h_table_f
 from sparsetriton_b200.tensor import SparseTensor, TensorCache
-from sparsetriton_b200.utils.hash import HashTable, round_up_capacity
+from sparsetriton_b200.utils.hash import HashTable
 
 from .funcs import ConvHashOnTheFlyImplicitGEMM, ConvPrecomputedNeighborGEMM
 from .funcs.implicit_precomputed_gemm import prepare_plans
-from .kmap import PendingOutCoordsAndMap, build_out_coords, kernel_offsets, out_coords_and_map
+from .kmap import PendingOutCoordsAndMap, _run_out_coords, kernel_offsets, output_shape
 
 __all__ = ["compute_neighbor_indices", "sparse_conv3d", "prepare_conv3d", "ConvPreparation"]
 
@@ -39,70 +39,38 @@ def compute_neighbor_indices(
     One kernel launch; the (N_out*K, 4) candidate rows of the reference are never materialised.
     """
     n_out, K = out_coords.shape[0], kernel_offsets.shape[0]
-    device = out_coords.device
-    nbr = torch.empty((n_out, K), dtype=torch.int32, device=device)
     if n_out == 0:
-        return nbr
+        return torch.empty((n_out, K), dtype=torch.int32, device=out_coords.device)
     _lib.require_cuda(out_coords, "compute_neighbor_indices")
     keys, vals = in_hash_table.table_keys, in_hash_table.table_values
     _lib.require_cuda(keys, "compute_neighbor_indices")
     if keys.dtype != torch.int64 or vals.dtype != torch.int32:
         raise TypeError("hash table must hold int64 keys and int32 values")
-    coords = out_coords.contiguous()
     host = getattr(kernel_offsets, "_st_host", None)
     if host is None:
         host = kernel_offsets.reshape(-1).tolist()
-    # Submanifold layer (the queries are the rows the table was built from, stride 1, odd kernel): offsets
-    # come in opposite pairs, so half of the probes give the whole map (no reference counterpart).
-    if queries_are_table_rows and int(stride) == 1 and K % 2 == 1 and \
-            all(host[i] == -host[3 * (K - 1) - 3 * (i // 3) + i % 3] for i in range(3 * K)):
-        with _lib.on_device(device), trace.stage("map_build", 3):
-            asym = torch.empty(1, dtype=torch.int32, device=device)
-            rc = _lib.lib().st_map_build_symmetric(_lib.ptr(coords), n_out, _lib.coord_code(coords), _lib.host_i32(host),
-                                                   K, _lib.host_i32(int(v) for v in spatial_shape), _lib.ptr(keys),
-                                                   _lib.ptr(vals), keys.shape[0], _lib.ptr(nbr), _lib.ptr(asym),
-                                                   _lib.stream_ptr())
-        _lib.check(rc, "st_map_build_symmetric")
-        # rows not returned for their own coordinate (duplicates, outside the grid); 0 = the map is its own
-        # inverse up to the order of the offsets, which the feature gradient then exploits.  The count travels to
-        # pinned host memory right away and an event marks its arrival, so that the backward pass, much later,
-        # reads it without waiting for everything the stream holds by then.
-        flag_host = torch.empty(1, dtype=torch.int32, pin_memory=True)
-        flag_host.copy_(asym, non_blocking=True)
-        arrived = torch.cuda.Event()
-        arrived.record(torch.cuda.current_stream(device))
-        nbr._st_asymmetric_rows = (flag_host, arrived)
-        return nbr
-    with _lib.on_device(device), trace.stage("map_build", 1):
-        rc = _lib.lib().st_map_build(_lib.ptr(coords), n_out, _lib.coord_code(coords), _lib.host_i32(host), K,
-                                     int(stride), _lib.host_i32(int(v) for v in spatial_shape), _lib.ptr(keys),
-                                     _lib.ptr(vals), keys.shape[0], _lib.ptr(nbr), _lib.stream_ptr())
-    _lib.check(rc, "st_map_build")
+    nbr, state = _lib.host().probe_map(out_coords, host, [int(v) for v in spatial_shape], int(stride), keys, vals,
+                                       bool(queries_are_table_rows))
+    # for a submanifold map the state also learns whether every row was found under its own coordinate: then the map is
+    # its own inverse up to the order of the offsets, which the feature gradient exploits
+    nbr._st_map = state
     return nbr
 
 
-def _new_table(coords, device):
-    table = HashTable(round_up_capacity(coords.shape[0], get_h_table_f()), device=device)
-    table.insert(coords)
-    return table
+def _new_table(coords):
+    return HashTable._built(*_lib.host().build_table(coords, get_h_table_f()))
 
 
-def _table_and_out_coords(cache, coords, spatial_shape, k, s, p, d, submanifold, transposed):
-    """Table over the coordinates the lookup is made in (the inputs themselves, or, for an upsampling transposed
-    conv, the inputs with their spatial columns scaled: conv.py:138-142) and the output coordinates."""
-    device = coords.device
+def _lookup_table(cache, coords, s, transposed):
+    """Table over the coordinates a hash-on-the-fly layer looks up: the inputs themselves, or, for an upsampling
+    transposed conv, the inputs with their spatial columns scaled (conv.py:138-142)."""
     if transposed and s > 1:
         scaled = coords.clone()
         scaled[:, 1:] *= s
-        table = _new_table(scaled, device)
-    else:
-        if cache.hashtable is None:
-            cache.hashtable = _new_table(coords, device)
-        table = cache.hashtable
-    out_coords, new_shape, koff = build_out_coords(coords, spatial_shape, k, s, d, p, transposed=transposed,
-                                                   submanifold=submanifold)
-    koff._st_host = [v for o in kernel_offsets(k, d, p, transposed) for v in o]
-    return table, out_coords, new_shape, koff
+        return _new_table(scaled)
+    if cache.hashtable is None:
+        cache.hashtable = _new_table(coords)
+    return cache.hashtable
 
 
 def _stored_geometry(cache, coords, spatial_shape, k, s, p, d, submanifold, transposed, batch_bound=0):
@@ -115,15 +83,18 @@ def _stored_geometry(cache, coords, spatial_shape, k, s, p, d, submanifold, tran
     if not (submanifold and s == 1):
         # strided / transposed layer: coordinates and map come out of one pass over the candidates; no table over
         # the inputs is needed
-        out_coords, new_shape, _, neighbor_indices = out_coords_and_map(coords, spatial_shape, k, s, d, p, transposed,
-                                                                        batch_bound)
+        out_coords, new_shape, neighbor_indices = PendingOutCoordsAndMap(coords, spatial_shape, k, s, d, p, transposed,
+                                                                         batch_bound).finish_map()
     else:
-        table, out_coords, new_shape, koff = _table_and_out_coords(cache, coords, spatial_shape, k, s, p, d,
-                                                                   submanifold, transposed)
-        upsample = transposed and s > 1
-        lookup_shape = tuple(v * s for v in spatial_shape) if upsample else tuple(spatial_shape)
-        neighbor_indices = compute_neighbor_indices(table, out_coords, koff, lookup_shape, 1 if transposed else s, p, d,
-                                                    queries_are_table_rows=out_coords is coords)
+        _lib.require_cuda(coords, "sparse_conv3d")
+        table = cache.hashtable
+        keys, vals, status, neighbor_indices, state = _lib.host().submanifold(
+            coords, spatial_shape, k, d, get_h_table_f(), table.table_keys if table is not None else None,
+            table.table_values if table is not None else None)
+        if table is None:
+            cache.hashtable = HashTable._built(keys, vals, status)
+        neighbor_indices._st_map = state
+        out_coords, new_shape = coords, spatial_shape
     if out_coords.shape[0] > 0:
         cache.neighbor_indices[cache_key] = (out_coords, neighbor_indices, new_shape)
     return out_coords, neighbor_indices, new_shape
@@ -171,7 +142,7 @@ class ConvPreparation:
         cache, coords = self.cache, self.coords
         with torch.cuda.stream(self.stream):
             if self.pending is not None:
-                out_coords, new_shape, _, nbr = self.pending.finish()
+                out_coords, new_shape, nbr = self.pending.finish_map()
                 self.pending = None
                 if out_coords.shape[0] > 0:
                     cache.neighbor_indices[self.geometry] = (out_coords, nbr, new_shape)
@@ -208,6 +179,14 @@ def prepare_conv3d(
     coordinates, neighbour map and tile plans of the layer (no reference counterpart)."""
     return ConvPreparation(coords, spatial_shape, kernel_size, stride, dilation, padding, transposed, submanifold,
                            backward, cache, consumer_stream, batch_size).finish()
+
+
+class _offsets:
+    """The (K, 3) offsets of a layer where only their host values are wanted."""
+
+    def __init__(self, k, d, p, transposed):
+        self._st_host = [v for o in kernel_offsets(k, d, p, transposed) for v in o]
+        self.shape = (k ** 3, 3)
 
 
 def _scalar(value, what):
@@ -251,14 +230,15 @@ def sparse_conv3d(
 
     cache = tensor._cache
     algo = get_conv_algo()
-    upsample = transposed and s > 1
-    neighbor_indices = table = koff = None
+    neighbor_indices = None
     if algo == ConvAlgo.PrecomputedNeighborGEMM:
         out_coords, neighbor_indices, new_shape = _stored_geometry(cache, coords, tensor.spatial_shape, k, s, p, d,
                                                                    submanifold, transposed, tensor.batch_size)
+    elif submanifold and s == 1:
+        out_coords, new_shape = coords, tensor.spatial_shape
     else:
-        table, out_coords, new_shape, koff = _table_and_out_coords(cache, coords, tensor.spatial_shape, k, s, p, d,
-                                                                   submanifold, transposed)
+        new_shape = output_shape(tensor.spatial_shape, k, s, d, p, transposed)
+        out_coords, _ = _run_out_coords(coords, k, d, p, new_shape, s, transposed, False, tensor.spatial_shape, tensor.batch_size)
 
     if out_coords.shape[0] == 0:
         return SparseTensor(
@@ -269,10 +249,12 @@ def sparse_conv3d(
     if algo == ConvAlgo.PrecomputedNeighborGEMM:
         out_feats = ConvPrecomputedNeighborGEMM.apply(feats, weight, neighbor_indices)
     elif algo == ConvAlgo.ImplicitHashFlyGEMM:
+        upsample = transposed and s > 1
+        table = _lookup_table(cache, coords, s, transposed)
         lookup_shape = tuple(v * s for v in tensor.spatial_shape) if upsample else tuple(tensor.spatial_shape)
-        lookup_stride = 1 if transposed else s
-        out_feats = ConvHashOnTheFlyImplicitGEMM.apply(feats, weight, out_coords, koff, table.table_keys,
-                                                       table.table_values, lookup_shape, lookup_stride)
+        out_feats = ConvHashOnTheFlyImplicitGEMM.apply(feats, weight, out_coords, _offsets(k, d, p, transposed),
+                                                       table.table_keys, table.table_values, lookup_shape,
+                                                       1 if transposed else s)
     else:  # pragma: no cover - ConvAlgo has two members
         raise ValueError(f"unknown convolution algorithm {algo}")
 

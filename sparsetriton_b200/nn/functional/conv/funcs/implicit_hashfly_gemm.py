@@ -26,34 +26,35 @@ import torch
 
 from sparsetriton_b200 import _lib, trace
 
-from sparsetriton_b200.config import get_hashfly_transient_map
+from sparsetriton_b200.config import get_hashfly_transient_map, get_row_order
 
 from ._channels import pad_cols, pad_weight, padded_widths
-from .implicit_precomputed_gemm import stored_map_dgrad, stored_map_forward, stored_map_wgrad
 
 __all__ = ["ConvHashOnTheFlyImplicitGEMM"]
 
 
 def _host_offsets(kernel_offsets):
+    """The (K,3) offsets as a flat host list."""
     host = getattr(kernel_offsets, "_st_host", None)
-    if host is None:
-        host = [int(v) for v in kernel_offsets.reshape(-1).tolist()]
-    return _lib.host_i32(host)
-
-
-def _probe_map(c, offsets_h, keys, vals, shape_h, lookup_stride, K):
-    """(N_out, K) int32 scratch map: row of (batch, out*stride - off[k]) in the table, or -1 (st_map_build)."""
-    n_out = c.shape[0]
-    nbr = torch.empty((n_out, K), dtype=torch.int32, device=c.device)
-    if n_out > 0:
-        with _lib.on_device(c.device), trace.stage("hashfly_probe", 1):
-            rc = _lib.lib().st_map_build(_lib.ptr(c), n_out, _lib.coord_code(c), offsets_h, K, lookup_stride, shape_h,
-                                         _lib.ptr(keys), _lib.ptr(vals), keys.shape[0], _lib.ptr(nbr), _lib.stream_ptr())
-        _lib.check(rc, "st_map_build")
-    return nbr
+    return host if host is not None else [int(v) for v in kernel_offsets.reshape(-1).tolist()]
 
 
 class ConvHashOnTheFlyImplicitGEMM(torch.autograd.Function):
+    @classmethod
+    def apply(cls, features, weights, coords, kernel_offsets, hash_table_keys, hash_table_vals, spatial_shape, lookup_stride):
+        if not get_hashfly_transient_map():
+            return super().apply(features, weights, coords, kernel_offsets, hash_table_keys, hash_table_vals, spatial_shape,
+                                 lookup_stride)
+        # the transient form is native (host/conv.cpp)
+        _lib.require_cuda(features, "ConvHashOnTheFlyImplicitGEMM")
+        K, w_cin, _ = weights.shape
+        assert w_cin == features.shape[1], f"weights expect {w_cin} input channels, features have {features.shape[1]}"
+        assert kernel_offsets.shape[0] == K, "kernel_offsets must be (K, 3)"
+        if hash_table_keys.dtype != torch.int64 or hash_table_vals.dtype != torch.int32:
+            raise TypeError("hash table must hold int64 keys and int32 values")
+        return _lib.host().conv_hashfly(features, weights, coords, _host_offsets(kernel_offsets), hash_table_keys, hash_table_vals,
+                                        [int(v) for v in spatial_shape], int(lookup_stride), get_row_order())
+
     @staticmethod
     def forward(ctx, features, weights, coords, kernel_offsets, hash_table_keys, hash_table_vals, spatial_shape,
                 lookup_stride):
@@ -71,18 +72,11 @@ class ConvHashOnTheFlyImplicitGEMM(torch.autograd.Function):
         w = pad_weight(weights.to(x.dtype), c_in, c_out).contiguous()
         c = coords.contiguous()
         keys, vals = hash_table_keys.contiguous(), hash_table_vals.contiguous()
-        ctx.offsets_h = _host_offsets(kernel_offsets)
+        ctx.offsets_h = _lib.host_i32(_host_offsets(kernel_offsets))
         ctx.shape_h = _lib.host_i32(int(v) for v in spatial_shape)
         ctx.lookup_stride = int(lookup_stride)
         ctx.w_dtype = weights.dtype
         code = _lib.feat_code(x)
-        ctx.transient = bool(get_hashfly_transient_map())
-        if ctx.transient:
-            nbr = _probe_map(c, ctx.offsets_h, keys, vals, ctx.shape_h, ctx.lookup_stride, K)
-            y, _ = stored_map_forward(x, w, nbr, n_in)
-            del nbr                                                   # the map and its plan die with the call
-            ctx.save_for_backward(x, w, c, keys, vals)
-            return y if c_out == ctx.true_widths[1] else y[:, :ctx.true_widths[1]].contiguous()
         y = torch.empty((n_out, c_out), device=x.device, dtype=x.dtype)
         if n_out > 0:
             with _lib.on_device(x.device), trace.stage("conv_fwd_hashfly", 1):
@@ -105,18 +99,6 @@ class ConvHashOnTheFlyImplicitGEMM(torch.autograd.Function):
         code, ccode = _lib.feat_code(x), _lib.coord_code(c)
         L = _lib.lib()
         dx = dw = None
-        if ctx.transient:
-            nbr = _probe_map(c, ctx.offsets_h, keys, vals, ctx.shape_h, ctx.lookup_stride, K)
-            if ctx.needs_input_grad[0]:
-                dx = stored_map_dgrad(dy, w, nbr, n_in)
-            if ctx.needs_input_grad[1]:
-                dw = stored_map_wgrad(x, dy, nbr, K).to(ctx.w_dtype)
-            del nbr
-            if dx is not None and t_in != c_in:
-                dx = dx[:, :t_in].contiguous()
-            if dw is not None and (t_in != c_in or t_out != c_out):
-                dw = dw[:, :t_in, :t_out].contiguous()
-            return dx, dw, None, None, None, None, None, None
         with _lib.on_device(x.device):
             stream = _lib.stream_ptr()
             ws = _lib.workspace(L.st_conv_hashfly_workspace_bytes(code, n_in, n_out, K, c_in, c_out), x.device)

@@ -16,11 +16,9 @@ Two reference behaviours are intentionally not reproduced:
 """
 from typing import Tuple
 
-import ctypes
-
 import torch
 
-from sparsetriton_b200 import _lib, trace
+from sparsetriton_b200 import _lib
 
 __all__ = ["build_out_coords", "out_coords_and_map", "PendingOutCoordsAndMap", "kernel_offsets", "output_shape"]
 
@@ -95,7 +93,7 @@ def build_out_coords(
 
     new_shape_t = _constant_tensor(new_shape, torch.int64, device, (3,)).clone()
     new_shape_t._st_host = new_shape      # spares callers in this package a device->host read
-    out, _ = _run_out_coords(in_coords, offsets, new_shape, stride, transposed, with_map=False)
+    out, _ = _run_out_coords(in_coords, kernel_size, dilation, padding, new_shape, stride, transposed, with_map=False)
     return out, new_shape_t, koff
 
 
@@ -110,80 +108,21 @@ def out_coords_and_map(in_coords, spatial_shape, kernel_size, stride, dilation, 
                                   batch_bound).finish()
 
 
-class _PendingOutCoords:
-    """First half of the output-coordinate build: candidates counted and deduplicated on the stream current at
-    construction, the count on its way to pinned host memory.  `finish()` waits for that copy alone (not for the
-    stream), sizes the outputs and launches the second half on the same stream."""
+def _run_out_coords(in_coords, kernel_size, dilation, padding, new_shape, stride, transposed, with_map, in_shape=(0, 0, 0),
+                    batch_bound=0):
+    """(out_coords, nbr or None) of a strided / transposed layer, through the native two-pass build."""
+    return _begin_out_coords(in_coords, kernel_size, dilation, padding, new_shape, stride, transposed, with_map, in_shape,
+                             batch_bound).finish()[:2]
 
-    def __init__(self, in_coords, offsets, new_shape, stride, transposed, with_map, in_shape=None, batch_bound=0):
-        device = in_coords.device
-        self.batch_bound = int(batch_bound or 0)   # samples in the batch if known: lets the library address cells directly
-        self.n, self.K = in_coords.shape[0], len(offsets)
-        self.with_map, self.coord_dtype, self.device = with_map, in_coords.dtype, device
-        if self.n == 0:
-            return
+
+def _begin_out_coords(in_coords, kernel_size, dilation, padding, new_shape, stride, transposed, with_map, in_shape, batch_bound):
+    """First half: candidates counted and deduplicated on the current stream, the count on its way to pinned host
+    memory.  `.finish()` waits for that alone (not for the stream), sizes the outputs, launches the second half on the same
+    stream and returns (out_coords, nbr, state of the map)."""
+    if in_coords.shape[0] > 0:
         _lib.require_cuda(in_coords, "build_out_coords")
-        self.coords = in_coords.contiguous()
-        self.code = _lib.coord_code(self.coords)
-        L = _lib.lib()
-        self.off_h = _lib.host_i32(v for o in offsets for v in o)
-        self.shape_h = _lib.host_i32(new_shape)
-        self.in_shape_h = _lib.host_i32(in_shape) if in_shape is not None else None
-        self.stride, self.transposed = stride, int(transposed)
-        self.ws = _lib.workspace(L.st_outcoords_workspace_bytes(self.n, self.K, stride, self.transposed), device)
-        self.counters = torch.zeros(2, dtype=torch.int64, device=device)      # [n_out, status]
-        self.status = self.counters[1:].view(torch.int32)
-        self.stream = torch.cuda.current_stream(device)
-        with _lib.on_device(device), trace.stage("out_coords"):
-            rc = L.st_outcoords_count(_lib.ptr(self.coords), self.n, self.code, self.off_h, self.K, stride,
-                                      self.transposed, self.shape_h, self.batch_bound, _lib.ptr(self.ws), self.ws.numel(),
-                                      _lib.ptr(self.counters), _lib.ptr(self.status), _lib.stream_ptr(device))
-            _lib.check(rc, "st_outcoords_count")
-            self.host = torch.empty(2, dtype=torch.int64, pin_memory=True)
-            self.host.copy_(self.counters, non_blocking=True)
-            # the tensor-core kernels' sticky status word rides along: this is the one wait a step makes anyway
-            self.kernel_status = torch.empty(4, dtype=torch.int32, pin_memory=True)
-            _lib.check(L.st_device_status_enqueue(ctypes.c_void_p(self.kernel_status.data_ptr()), _lib.stream_ptr(device)),
-                       "st_device_status_enqueue")
-            self.arrived = torch.cuda.Event()
-            self.arrived.record(self.stream)
-
-    def finish(self):
-        device, K = self.device, self.K
-        if self.n == 0:
-            return (torch.empty((0, 4), dtype=self.coord_dtype, device=device),
-                    torch.empty((0, K), dtype=torch.int32, device=device) if self.with_map else None)
-        L = _lib.lib()
-        self.arrived.synchronize()                                     # the one device->host wait
-        n_out, flags = self.host.tolist()
-        _lib.raise_on_timeout(self.kernel_status, device)
-        if flags & _lib.DEV_TABLE_FULL:
-            raise RuntimeError("build_out_coords: dedupe table overflow")
-        if flags & _lib.DEV_BAD_INDEX:
-            raise ValueError(f"build_out_coords: a batch index lies outside [0, {self.batch_bound}) (the batch size given)")
-        nbr = None
-        with _lib.on_device(device), torch.cuda.stream(self.stream):
-            stream = _lib.stream_ptr(device)
-            out = torch.empty((n_out, 4), dtype=self.coord_dtype, device=device)
-            if n_out > 0:
-                with trace.stage("out_coords"):
-                    rc = L.st_outcoords_write(_lib.ptr(self.coords), self.n, self.code, self.off_h, K, self.stride,
-                                              self.transposed, self.shape_h, self.batch_bound, _lib.ptr(self.ws), self.ws.numel(),
-                                              _lib.ptr(out), n_out, _lib.ptr(self.status), stream)
-                    _lib.check(rc, "st_outcoords_write")
-            if self.with_map:
-                nbr = torch.empty((n_out, K), dtype=torch.int32, device=device)
-                if n_out > 0:
-                    with trace.stage("map_scatter"):
-                        rc = L.st_outcoords_map(_lib.ptr(self.coords), self.n, self.code, self.off_h, K, self.stride,
-                                                self.transposed, self.shape_h, self.in_shape_h, self.batch_bound,
-                                                _lib.ptr(self.ws), self.ws.numel(), _lib.ptr(nbr), n_out, stream)
-                        _lib.check(rc, "st_outcoords_map")
-        return out, nbr
-
-
-def _run_out_coords(in_coords, offsets, new_shape, stride, transposed, with_map, in_shape=None, batch_bound=0):
-    return _PendingOutCoords(in_coords, offsets, new_shape, stride, transposed, with_map, in_shape, batch_bound).finish()
+    return _lib.host().OutCoords(in_coords, kernel_size, stride, dilation, padding, bool(transposed), list(new_shape),
+                                 [int(v) for v in in_shape], int(batch_bound or 0), with_map)
 
 
 class PendingOutCoordsAndMap:
@@ -191,13 +130,21 @@ class PendingOutCoordsAndMap:
     `out_coords_and_map` returns.  Lets a caller put other work between the launch and the wait for the count."""
 
     def __init__(self, in_coords, spatial_shape, kernel_size, stride, dilation, padding, transposed, batch_bound=0):
-        offsets = kernel_offsets(kernel_size, dilation, padding, transposed)
-        self.koff = _offsets_tensor(offsets, in_coords)
-        self.koff._st_host = [v for o in offsets for v in o]
+        self.geometry = (kernel_size, dilation, padding, transposed)
+        self.like = in_coords
         self.new_shape = output_shape(spatial_shape, kernel_size, stride, dilation, padding, transposed)
-        self.pending = _PendingOutCoords(in_coords, offsets, self.new_shape, stride, transposed, with_map=True,
-                                         in_shape=tuple(int(v) for v in spatial_shape), batch_bound=batch_bound)
+        self.pending = _begin_out_coords(in_coords, kernel_size, dilation, padding, self.new_shape, stride, transposed, True,
+                                         spatial_shape, batch_bound)
+
+    def finish_map(self):
+        """(out_coords, new_shape, nbr): `finish` without the offsets tensor."""
+        out, nbr, state = self.pending.finish()
+        nbr._st_map = state
+        return out, self.new_shape, nbr
 
     def finish(self):
-        out, nbr = self.pending.finish()
-        return out, self.new_shape, self.koff, nbr
+        out, new_shape, nbr = self.finish_map()
+        offsets = kernel_offsets(*self.geometry)
+        koff = _offsets_tensor(offsets, self.like)
+        koff._st_host = [v for o in offsets for v in o]
+        return out, new_shape, koff, nbr

@@ -9,6 +9,7 @@ from typing import Any, Dict, Optional, Tuple
 
 import torch
 
+from sparsetriton_b200 import _lib
 from sparsetriton_b200.config import get_coords_dtype
 from sparsetriton_b200.utils.hash import HashTable
 from sparsetriton_b200.utils.to_dense import to_dense
@@ -55,7 +56,10 @@ class SparseTensor:
 
         n = self.coords.shape[0]
         # one device->host transfer serves both derived quantities
-        extent = self.coords.max(dim=0).values.tolist() if n > 0 else None
+        extent = None
+        if n > 0:
+            on_device = self.coords.is_cuda and self.coords.dtype in (torch.int16, torch.int32)
+            extent = _lib.host().extent(self.coords) if on_device else self.coords.max(dim=0).values.tolist()
         if spatial_shape is None:
             self.spatial_shape = torch.Size([v + 1 for v in extent[1:]]) if n > 0 else torch.Size([0, 0, 0])
         else:

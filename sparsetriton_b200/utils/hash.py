@@ -66,6 +66,14 @@ class HashTable:
             self.table_keys = torch.full((capacity,), -1, dtype=torch.int64, device=dev)
             self.table_values = torch.full((capacity,), -1, dtype=torch.int32, device=dev)
 
+    @classmethod
+    def _built(cls, keys, vals, status):
+        """A table whose arrays the library has made and filled already; `status`: the words its builder reported into."""
+        self = cls(table_keys=keys, table_values=vals)
+        if status is not None:
+            self._status = status
+        return self
+
     @property
     def device(self):
         return self.table_keys.device
@@ -119,7 +127,7 @@ class HashTable:
         each of them passed on its own) or met a coordinate outside [0, 65535], which has no key.  One
         device->host read; no reference counterpart (the reference drops such keys silently)."""
         status = getattr(self, "_status", None)
-        flags = int(status.item()) if status is not None else 0
+        flags = int(status[0].item()) if status is not None else 0
         if flags & _lib.DEV_TABLE_FULL:
             raise RuntimeError("HashTable: an insert found no free slot (capacity too small for all inserted keys)")
         if flags & _lib.DEV_BAD_INDEX:
