@@ -166,6 +166,14 @@ int st_map_build_symmetric(const void* coords, int64_t n, int coord_dtype, const
                            const int32_t* lookup_shape_host, const int64_t* keys, const int32_t* vals, int64_t capacity,
                            int32_t* nbr, int32_t* asymmetric_rows, void* stream);
 
+/* The same with scratch: from half a million probes on, cubic offset sets of kernels 3, 5 and 7 are then looked up in a
+ * filter of occupied columns first, and in the row table only where a bit is set.  Same result.  _workspace_bytes is 0 where
+ * scratch would not be used; without it the call is st_map_build_symmetric. */
+int64_t st_map_build_symmetric_workspace_bytes(int64_t n, int K);
+int st_map_build_symmetric_ws(const void* coords, int64_t n, int coord_dtype, const int32_t* offsets_host, int K,
+                              const int32_t* lookup_shape_host, const int64_t* keys, const int32_t* vals, int64_t capacity,
+                              int32_t* nbr, int32_t* asymmetric_rows, void* workspace, int64_t workspace_bytes, void* stream);
+
 /* inv[i,k] = o for every nbr[o,k] = i >= 0, -1 elsewhere (inv is (n_in,K) and is fully written).
  * No counterpart in the reference, whose dgrad scatters with atomics
  * (funcs/implicit_precomputed_gemm.py:129-177); this is the map its gather-form dgrad reads. */

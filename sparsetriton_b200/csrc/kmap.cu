@@ -6,6 +6,8 @@
 // (rows, K) tables is coalesced; the output-coordinate kernels give each input row one thread that
 // loops over its K offsets.  Order-defining steps (which duplicate survives, where a row lands) are
 // functions of t only, so results do not depend on scheduling.
+#include <type_traits>
+
 #include "common.cuh"
 
 namespace st {
@@ -497,19 +499,60 @@ outcoords_map_kernel(const CT* __restrict__ coords, int64_t n, int K, Offsets of
   });
 }
 
+// The offsets of a cubic kernel, base + i * step per axis with k = (ix * ks + iy) * ks + iz.  Threads of one warp stand at
+// different k: reading a table of offsets from the launch parameters then costs one constant-cache access per distinct k
+// (map of 2 M random cells, ks = 5, by columns: 703 us with the table, 581 us computed).
+struct CubeOffsets {
+  int ks, base[3], step[3];
+  __device__ __forceinline__ int at(int axis, int i) const { return base[axis] + i * step[axis]; }
+};
+static bool cube_offsets(const int32_t* off, int K, CubeOffsets* out) {
+  for (int ks = 1; ks <= 7; ++ks) {
+    if (ks * ks * ks != K) continue;
+    out->ks = ks;
+    const int stride_k[3] = {ks * ks, ks, 1};
+    for (int a = 0; a < 3; ++a) {
+      out->base[a] = off[a];
+      out->step[a] = ks > 1 ? off[stride_k[a] * 3 + a] - off[a] : 0;
+    }
+    for (int k = 0; k < K; ++k)
+      for (int a = 0; a < 3; ++a)
+        if (off[k * 3 + a] != out->base[a] + k / stride_k[a] % ks * out->step[a]) return false;
+    return true;
+  }
+  return false;
+}
+// Offset k of either form.  KS: the kernel size when the offsets are a cube's (`cube`), 0: the table.
+template <int KS>
+__device__ __forceinline__ int3 offset_of(const Offsets& off, const CubeOffsets& cube, int k) {
+  if (KS == 0) return make_int3(off.v[k * 3 + 0], off.v[k * 3 + 1], off.v[k * 3 + 2]);
+  constexpr int D = KS > 0 ? KS : 1;
+  return make_int3(cube.at(0, k / (D * D)), cube.at(1, k / D % D), cube.at(2, k % D));
+}
+#define ST_BY_KERNEL_SIZE(cubic, cube, ...)                                                   \
+  do {                                                                                        \
+    if (!(cubic)) { constexpr int KS = 0; __VA_ARGS__; }                                      \
+    else if ((cube).ks == 2) { constexpr int KS = 2; __VA_ARGS__; }                           \
+    else if ((cube).ks == 3) { constexpr int KS = 3; __VA_ARGS__; }                           \
+    else if ((cube).ks == 5) { constexpr int KS = 5; __VA_ARGS__; }                           \
+    else { constexpr int KS = 0; __VA_ARGS__; }                                               \
+  } while (0)
+
 // nbr[o,k] = row of (b, out*stride - off[k]) or -1.
-template <typename CT>
+template <typename CT, int KS>
 __global__ void __launch_bounds__(256)
-map_build_kernel(const CT* __restrict__ out_coords, int64_t n_flat, int K, Offsets off, int stride, Int3 shape,
-                 Table table, int32_t* __restrict__ nbr) {
+map_build_kernel(const CT* __restrict__ out_coords, int64_t n_flat, int k_volume, Offsets off, CubeOffsets cube, int stride,
+                 Int3 shape, Table table, int32_t* __restrict__ nbr) {
   int64_t t = (int64_t)blockIdx.x * 256 + threadIdx.x;
   if (t >= n_flat) return;
-  int64_t row = t / K;
+  const int K = KS > 0 ? KS * KS * KS : k_volume;
+  int64_t row = n_flat <= 0xFFFFFFFFll ? (int64_t)((uint32_t)t / (uint32_t)K) : t / K;
   int k = (int)(t - row * K);
   int4 c = load_coord<CT>(out_coords, row);
-  int x = c.y * stride - off.v[k * 3 + 0];
-  int y = c.z * stride - off.v[k * 3 + 1];
-  int z = c.w * stride - off.v[k * 3 + 2];
+  const int3 o = offset_of<KS>(off, cube, k);
+  int x = c.y * stride - o.x;
+  int y = c.z * stride - o.y;
+  int z = c.w * stride - o.z;
   int32_t r = -1;
   if (x >= 0 && x < shape.x && y >= 0 && y < shape.y && z >= 0 && z < shape.z && table.capacity != 0 &&
       key_representable(c.x, x, y, z))
@@ -522,17 +565,19 @@ map_build_kernel(const CT* __restrict__ out_coords, int64_t n_flat, int K, Offse
 // neighbour of o at k" means "o is the neighbour of i at K-1-k": a thread probes offset k <= K/2 of its
 // row, stores the hit, and mirrors it with atomicMax (the table's own rule for duplicate coordinates:
 // the largest row wins).  nbr must hold -1 in its upper half.
-template <typename CT>
+template <typename CT, int KS>
 __global__ void __launch_bounds__(256)
-map_build_half_kernel(const CT* __restrict__ coords, int64_t n_half, int K, Offsets off, Int3 shape, Table table,
-                      int32_t* __restrict__ nbr) {
+map_build_half_kernel(const CT* __restrict__ coords, int64_t n_half, int k_volume, Offsets off, CubeOffsets cube, Int3 shape,
+                      Table table, int32_t* __restrict__ nbr) {
   const int64_t t = (int64_t)blockIdx.x * 256 + threadIdx.x;
   if (t >= n_half) return;
+  const int K = KS > 0 ? KS * KS * KS : k_volume;
   const int half = K / 2 + 1;
-  const int64_t row = t / half;
+  const int64_t row = n_half <= 0xFFFFFFFFll ? (int64_t)((uint32_t)t / (uint32_t)half) : t / half;
   const int k = (int)(t - row * half);
   const int4 c = load_coord<CT>(coords, row);
-  const int x = c.y - off.v[k * 3 + 0], y = c.z - off.v[k * 3 + 1], z = c.w - off.v[k * 3 + 2];
+  const int3 o = offset_of<KS>(off, cube, k);
+  const int x = c.y - o.x, y = c.z - o.y, z = c.w - o.z;
   int32_t r = -1;
   if (x >= 0 && x < shape.x && y >= 0 && y < shape.y && z >= 0 && z < shape.z && table.capacity != 0 &&
       key_representable(c.x, x, y, z))
@@ -542,6 +587,71 @@ map_build_half_kernel(const CT* __restrict__ coords, int64_t n_half, int K, Offs
   // the mirrored entry looks this row's own coordinate up, which the probing form bounds-checks
   if (c.y < 0 || c.y >= shape.x || c.z < 0 || c.z >= shape.y || c.w < 0 || c.w >= shape.z) return;
   atomicMax(nbr + (int64_t)r * K + (K - 1 - k), (int32_t)row);
+}
+
+// The same map behind a filter.  Of the half of the offsets that is probed most miss (13 of 14 for cells scattered in a large
+// grid, 10 of 14 on surfaces), and a probe that misses costs a random 32-byte sector of a large table like one that hits.
+// The filter has one 32-bit word per hashed column (b, x, y, z >> 5), with bit z & 31 set for every row: a row looks up the
+// ks*ks/2 + 1 columns of its half neighbourhood (5 words instead of 14 probes for ks = 3, 13 instead of 63 for ks = 5; two
+// where the z range straddles a block) and probes the row table only for bits that are set.  Columns that share a word only cause
+// probes that miss: with two words or more per row, one bit in 64 is set.  No keys and no chains: the build is one atomicOr per row.
+// 2 M random cells, clear and build included: ks = 3 0.55 -> 0.19 ms, ks = 5 2.96 -> 0.46 ms.
+struct ColumnFilter {
+  uint32_t* words;
+  uint32_t mask;                   // words - 1
+  __device__ __forceinline__ uint32_t* word(int b, int x, int y, int z) const {
+    return words + (mix_key(pack_key(b, x, y, z >> 5)) & mask);
+  }
+};
+
+template <typename CT>
+__global__ void __launch_bounds__(256) columns_build_kernel(const CT* __restrict__ coords, int64_t n, ColumnFilter f) {
+  const int64_t i = (int64_t)blockIdx.x * 256 + threadIdx.x;
+  if (i >= n) return;
+  const int4 c = load_coord<CT>(coords, i);
+  if (key_representable(c.x, c.y, c.z, c.w)) atomicOr(f.word(c.x, c.y, c.z, c.w), 1u << (c.w & 31));
+}
+
+template <typename CT, int KS>
+__global__ void __launch_bounds__(256)
+map_build_columns_kernel(const CT* __restrict__ coords, int64_t n_threads, CubeOffsets cube, Int3 shape, Table table,
+                         ColumnFilter filter, int32_t* __restrict__ nbr) {
+  constexpr int K = KS * KS * KS, kCols = KS * KS / 2 + 1;
+  const int64_t t = (int64_t)blockIdx.x * 256 + threadIdx.x;
+  if (t >= n_threads) return;
+  const int64_t row = n_threads <= 0xFFFFFFFFll ? (int64_t)((uint32_t)t / (uint32_t)kCols) : t / kCols;
+  const int col = (int)(t - row * kCols), k0 = col * KS;
+  const int4 c = load_coord<CT>(coords, row);
+  const int x = c.y - cube.at(0, col / KS), y = c.z - cube.at(1, col % KS);
+  if (x < 0 || x >= shape.x || y < 0 || y >= shape.y || table.capacity == 0 || !key_representable(c.x, x, y, 0)) return;
+  const int last = col == kCols - 1 ? KS / 2 : KS - 1;         // the centre column: up to the row itself
+  const bool inside = c.y >= 0 && c.y < shape.x && c.z >= 0 && c.z < shape.y && c.w >= 0 && c.w < shape.z;
+  int have = -1;                                               // block whose bits are at hand
+  uint32_t bits = 0;
+#pragma unroll
+  for (int iz = 0; iz < KS; ++iz) {
+    const int z = c.w - cube.at(2, iz);
+    if (iz > last || z < 0 || z >= shape.z || z > 0xFFFF) continue;
+    if ((z >> 5) != have) {
+      have = z >> 5;
+      bits = __ldg(filter.word(c.x, x, y, z));
+    }
+    if (!((bits >> (z & 31)) & 1u)) continue;
+    const int32_t r = table_find(table, pack_key(c.x, x, y, z));
+    if (r < 0) continue;
+    const int k = k0 + iz;
+    nbr[row * K + k] = r;
+    // the mirrored entry looks this row's own coordinate up, which the probing form bounds-checks
+    if (k != K / 2 && inside) atomicMax(nbr + (int64_t)r * K + (K - 1 - k), (int32_t)row);
+  }
+}
+
+// Probes from which the filter pays for its clear and build (two launches more).
+constexpr int64_t kFilterProbes = 1 << 19;
+static int64_t filter_words(int64_t n) {
+  int64_t words = 1024;
+  while (words < 2 * n) words <<= 1;
+  return words;
 }
 
 // Rows that the table does not return for their own coordinate (smaller duplicates, coordinates outside
@@ -1104,22 +1214,39 @@ int st_map_build(const void* out_coords, int64_t n_out, int coord_dtype, const i
   int64_t n_flat = n_out * K;
   unsigned grid = (unsigned)((n_flat + 255) / 256);
   cudaStream_t s = (cudaStream_t)stream;
-  if (coord_dtype == ST_I32)
-    { map_build_kernel<int32_t><<<grid, 256, 0, s>>>(static_cast<const int32_t*>(out_coords), n_flat, K, off,
-                                                   lookup_stride, shape, t, nbr); note_launches(1); }
-  else if (coord_dtype == ST_I16)
-    { map_build_kernel<int16_t><<<grid, 256, 0, s>>>(static_cast<const int16_t*>(out_coords), n_flat, K, off,
-                                                   lookup_stride, shape, t, nbr); note_launches(1); }
-  else {
+  if (coord_dtype != ST_I32 && coord_dtype != ST_I16) {
     set_error("st_map_build: unknown coordinate dtype %d", coord_dtype);
     return ST_ERR_DTYPE;
   }
+  CubeOffsets cube{};
+  const bool cubic = cube_offsets(offsets_host, K, &cube);
+  ST_BY_KERNEL_SIZE(cubic, cube, {
+    if (coord_dtype == ST_I32)
+      map_build_kernel<int32_t, KS><<<grid, 256, 0, s>>>(static_cast<const int32_t*>(out_coords), n_flat, K, off, cube, lookup_stride,
+                                                         shape, t, nbr);
+    else
+      map_build_kernel<int16_t, KS><<<grid, 256, 0, s>>>(static_cast<const int16_t*>(out_coords), n_flat, K, off, cube, lookup_stride,
+                                                         shape, t, nbr);
+  });
+  note_launches(1);
   return check_launch("st_map_build");
 }
 
 int st_map_build_symmetric(const void* coords, int64_t n, int coord_dtype, const int32_t* offsets_host, int K,
                            const int32_t* lookup_shape_host, const int64_t* keys, const int32_t* vals, int64_t capacity,
                            int32_t* nbr, int32_t* asymmetric_rows, void* stream) {
+  return st_map_build_symmetric_ws(coords, n, coord_dtype, offsets_host, K, lookup_shape_host, keys, vals, capacity, nbr,
+                                   asymmetric_rows, nullptr, 0, stream);
+}
+
+int64_t st_map_build_symmetric_workspace_bytes(int64_t n, int K) {
+  if (n < 1 || K < 27 || n * (K / 2 + 1) < kFilterProbes) return 0;
+  return filter_words(n) * 4;
+}
+
+int st_map_build_symmetric_ws(const void* coords, int64_t n, int coord_dtype, const int32_t* offsets_host, int K,
+                              const int32_t* lookup_shape_host, const int64_t* keys, const int32_t* vals, int64_t capacity,
+                              int32_t* nbr, int32_t* asymmetric_rows, void* workspace, int64_t workspace_bytes, void* stream) {
   if (n < 0 || K < 1 || K > ST_MAX_KVOL || (K & 1) == 0 || !offsets_host || !lookup_shape_host || capacity < 0 ||
       capacity > 0x7FFFFFFFll || (n > 0 && (!coords || !nbr)) || (capacity > 0 && (!keys || !vals))) {
     set_error("st_map_build_symmetric: bad arguments (K must be odd)");
@@ -1147,17 +1274,42 @@ int st_map_build_symmetric(const void* coords, int64_t n, int coord_dtype, const
   const Table t = make_table(keys, vals, capacity);
   const int64_t n_flat = n * K, n_half = n * (K / 2 + 1);
   cudaMemsetAsync(nbr, 0xFF, (size_t)n_flat * sizeof(int32_t), s);                             // every entry -1
-  if (coord_dtype == ST_I32) {
-    map_build_half_kernel<int32_t><<<(unsigned)((n_half + 255) / 256), 256, 0, s>>>(static_cast<const int32_t*>(coords),
-                                                                                   n_half, K, off, shape, t, nbr);
-    map_build_rest_kernel<int32_t><<<(unsigned)((n + 255) / 256), 256, 0, s>>>(static_cast<const int32_t*>(coords), n, K,
-                                                                              off, shape, t, nbr, asymmetric_rows);
-  } else {
-    map_build_half_kernel<int16_t><<<(unsigned)((n_half + 255) / 256), 256, 0, s>>>(static_cast<const int16_t*>(coords),
-                                                                                   n_half, K, off, shape, t, nbr);
-    map_build_rest_kernel<int16_t><<<(unsigned)((n + 255) / 256), 256, 0, s>>>(static_cast<const int16_t*>(coords), n, K,
-                                                                              off, shape, t, nbr, asymmetric_rows);
+  CubeOffsets cube{};
+  const bool cubic = cube_offsets(offsets_host, K, &cube);
+  const int ks = cubic && (cube.ks == 3 || cube.ks == 5 || cube.ks == 7) ? cube.ks : 0;
+  const int64_t need = st_map_build_symmetric_workspace_bytes(n, K);
+  if (ks && need > 0 && workspace && workspace_bytes >= need && (reinterpret_cast<uintptr_t>(workspace) & 15) == 0) {
+    const int64_t words = filter_words(n);
+    const ColumnFilter filter{static_cast<uint32_t*>(workspace), (uint32_t)(words - 1)};
+    cudaMemsetAsync(filter.words, 0, (size_t)words * 4, s);
+    const int64_t threads = n * (ks * ks / 2 + 1);
+    const unsigned grid = (unsigned)((threads + 255) / 256), rows = (unsigned)((n + 255) / 256);
+    auto sweep = [&](auto* typed) {
+      using CT = std::remove_const_t<std::remove_pointer_t<decltype(typed)>>;
+      columns_build_kernel<CT><<<rows, 256, 0, s>>>(typed, n, filter);
+      if (ks == 3) map_build_columns_kernel<CT, 3><<<grid, 256, 0, s>>>(typed, threads, cube, shape, t, filter, nbr);
+      else if (ks == 5) map_build_columns_kernel<CT, 5><<<grid, 256, 0, s>>>(typed, threads, cube, shape, t, filter, nbr);
+      else map_build_columns_kernel<CT, 7><<<grid, 256, 0, s>>>(typed, threads, cube, shape, t, filter, nbr);
+      map_build_rest_kernel<CT><<<rows, 256, 0, s>>>(typed, n, K, off, shape, t, nbr, asymmetric_rows);
+    };
+    if (coord_dtype == ST_I32) sweep(static_cast<const int32_t*>(coords));
+    else sweep(static_cast<const int16_t*>(coords));
+    note_launches(3);
+    return check_launch("st_map_build_symmetric");
   }
+  const unsigned half_grid = (unsigned)((n_half + 255) / 256), rows = (unsigned)((n + 255) / 256);
+  ST_BY_KERNEL_SIZE(cubic, cube, {
+    if (coord_dtype == ST_I32)
+      map_build_half_kernel<int32_t, KS><<<half_grid, 256, 0, s>>>(static_cast<const int32_t*>(coords), n_half, K, off, cube, shape, t,
+                                                                   nbr);
+    else
+      map_build_half_kernel<int16_t, KS><<<half_grid, 256, 0, s>>>(static_cast<const int16_t*>(coords), n_half, K, off, cube, shape, t,
+                                                                   nbr);
+  });
+  if (coord_dtype == ST_I32)
+    map_build_rest_kernel<int32_t><<<rows, 256, 0, s>>>(static_cast<const int32_t*>(coords), n, K, off, shape, t, nbr, asymmetric_rows);
+  else
+    map_build_rest_kernel<int16_t><<<rows, 256, 0, s>>>(static_cast<const int16_t*>(coords), n, K, off, shape, t, nbr, asymmetric_rows);
   note_launches(2);
   return check_launch("st_map_build_symmetric");
 }

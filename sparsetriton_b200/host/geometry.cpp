@@ -139,6 +139,9 @@ std::vector<int32_t> kernel_offsets(int k, int d, int p, bool transposed) {
 std::tuple<Tensor, Tensor, Tensor> build_table(const Tensor& coords_in, double factor) {
   const Tensor coords = coords_in.contiguous();
   const int64_t n = coords.size(0);
+  // In a small table the longest run of occupied slots, walked by dependent atomics, is what the insert waits for: twice the
+  // slots for up to 64 k rows (4096 rows: 13 -> 6 us).
+  if (n <= 65536) factor *= 2;
   int64_t want = (int64_t)((double)n * factor), capacity = 1;
   while (capacity < want) capacity <<= 1;
   const c10::cuda::OptionalCUDAGuard guard(coords.device());
@@ -179,9 +182,11 @@ std::tuple<Tensor, MapPtr> probe_map(const Tensor& coords_in, const std::vector<
   Stage stage("map_build", s);
   if (mirrored) {
     Tensor asym = empty_like_on(coords, {1}, at::kInt);
-    check(st_map_build_symmetric(coords.data_ptr(), n, code, offsets.data(), K, shape.data(), keys.data_ptr<int64_t>(),
-                                 vals.data_ptr<int32_t>(), keys.size(0), nbr.data_ptr<int32_t>(), asym.data_ptr<int32_t>(), s),
-          "st_map_build_symmetric");
+    const int64_t bytes = st_map_build_symmetric_workspace_bytes(n, K);
+    Tensor ws = bytes > 0 ? bytes_on(coords, bytes) : Tensor();
+    check(st_map_build_symmetric_ws(coords.data_ptr(), n, code, offsets.data(), K, shape.data(), keys.data_ptr<int64_t>(),
+                                    vals.data_ptr<int32_t>(), keys.size(0), nbr.data_ptr<int32_t>(), asym.data_ptr<int32_t>(),
+                                    bytes > 0 ? ws.data_ptr() : nullptr, bytes, s), "st_map_build_symmetric");
     state->expect_flag(nbr, asym.data_ptr<int32_t>(), s);
   } else {
     check(st_map_build(coords.data_ptr(), n, code, offsets.data(), K, stride, shape.data(), keys.data_ptr<int64_t>(),

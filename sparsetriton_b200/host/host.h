@@ -173,5 +173,8 @@ Tensor batch_norm_train(const Tensor& x, const c10::optional<Tensor>& w, const c
 Tensor batch_norm_running(const Tensor& x, const c10::optional<Tensor>& w, const c10::optional<Tensor>& b, const Tensor& mean,
                           const Tensor& var, double eps, bool relu);
 Tensor concat_cols(const Tensor& left, const Tensor& right);
+std::vector<Tensor> pool(const Tensor& feats, const Tensor& coords, std::vector<int64_t> shape, int64_t kernel, int64_t padding,
+                         int64_t stride, bool max, int64_t batch);
+Tensor to_dense(const Tensor& feats, const Tensor& coords, std::vector<int64_t> shape, int64_t batch);
 
 }  // namespace st_host

@@ -70,6 +70,8 @@ PYBIND11_MODULE(_st_host, m) {
   m.def("batch_norm_train", &batch_norm_train, Release());
   m.def("batch_norm_running", &batch_norm_running, Release());
   m.def("concat_cols", &concat_cols, Release());
+  m.def("pool", &pool, Release());
+  m.def("to_dense", &to_dense, Release());
   m.def("trace_start", &trace_start);
   m.def("trace_stop", &trace_stop);
   m.def("trace_spans", &trace_spans, Release());

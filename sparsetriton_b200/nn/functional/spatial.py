@@ -23,8 +23,10 @@ __all__ = ["sparse_pooling", "sparse_upsample", "SparsePoolingFunction", "Sparse
 
 
 class SparsePoolingFunction(torch.autograd.Function):
+    """`apply` makes the native node (host/spatial.cpp)."""
+
     @staticmethod
-    def forward(ctx, in_feats, in_coords, spatial_shape, kernel_size, padding, stride, mode="max", batch_size=None):
+    def apply(in_feats, in_coords, spatial_shape, kernel_size, padding, stride, mode="max", batch_size=None):
         if mode not in ("max", "avg"):
             raise ValueError(f"Unsupported mode: {mode}")
         _lib.require_cuda(in_feats, "sparse_pooling")
@@ -32,52 +34,11 @@ class SparsePoolingFunction(torch.autograd.Function):
             stride = kernel_size
         shape = tuple(int(v) for v in spatial_shape)
         new_shape = tuple((s - kernel_size + padding * 2) // stride + 1 for s in shape)          # spatial.py:116
-        feats = in_feats.contiguous()
-        coords = in_coords.contiguous()
-        dev = feats.device
-        n, C = feats.shape
         if batch_size is None:
-            batch_size = int(coords[:, 0].max().item()) + 1 if n > 0 else 0
-        L = _lib.lib()
-        code, ccode = _lib.feat_code(feats), _lib.coord_code(coords)
-        shape_h = _lib.host_i32(shape)
-        ws = _lib.workspace(L.st_pool_workspace_bytes(n), dev)
-        counters = torch.zeros(2, dtype=torch.int64, device=dev)          # [n_out, status]
-        status = counters[1:].view(torch.int32)
-        with _lib.on_device(dev), trace.stage("pool_map"):
-            s = _lib.stream_ptr()
-            _lib.check(L.st_pool_count(_lib.ptr(coords), n, ccode, kernel_size, padding, stride, shape_h, int(batch_size),
-                                       _lib.ptr(ws), ws.numel(), _lib.ptr(counters), _lib.ptr(status), s), "st_pool_count")
-            n_out, flags = counters.tolist()                               # the one device->host read
-            if flags & _lib.DEV_BAD_INDEX:
-                raise ValueError("sparse_pooling: a coordinate lies outside spatial_shape / batch_size")
-            out_coords = torch.empty((n_out, 4), dtype=coords.dtype, device=dev)
-            in_to_out = torch.empty((n,), dtype=torch.int32, device=dev)
-            members = torch.empty((n,), dtype=torch.int32, device=dev)
-            seg_start = torch.empty((n_out + 1,), dtype=torch.int32, device=dev)
-            _lib.check(L.st_pool_write(_lib.ptr(coords), n, ccode, kernel_size, padding, stride, shape_h, int(batch_size),
-                                       _lib.ptr(ws), ws.numel(), _lib.ptr(out_coords), n_out, _lib.ptr(in_to_out),
-                                       _lib.ptr(members), _lib.ptr(seg_start), s), "st_pool_write")
-        out_feats = torch.empty((n_out, C), dtype=feats.dtype, device=dev)
-        with _lib.on_device(dev), trace.stage("pool_fwd"):
-            _lib.check(L.st_pool_fwd(code, _lib.ptr(feats), C, _lib.ptr(members), _lib.ptr(seg_start), n_out,
-                                     int(mode == "max"), _lib.ptr(out_feats), _lib.stream_ptr()), "st_pool_fwd")
-        ctx.save_for_backward(feats, out_feats, in_to_out, seg_start)
-        ctx.mode = mode
-        ctx.mark_non_differentiable(out_coords)
+            batch_size = int(in_coords[:, 0].max().item()) + 1 if in_coords.shape[0] > 0 else 0
+        out_feats, out_coords = _lib.host().pool(in_feats, in_coords, shape, int(kernel_size), int(padding), int(stride),
+                                                 mode == "max", int(batch_size))
         return out_feats, out_coords, new_shape
-
-    @staticmethod
-    def backward(ctx, grad_out_feats, grad_out_coords, grad_spatial_shape):
-        feats, out_feats, in_to_out, seg_start = ctx.saved_tensors
-        n, C = feats.shape
-        g = grad_out_feats.to(feats.dtype).contiguous()
-        grad_in = torch.empty_like(feats)
-        with _lib.on_device(feats.device), trace.stage("pool_bwd"):
-            _lib.check(_lib.lib().st_pool_bwd(_lib.feat_code(feats), _lib.ptr(g), _lib.ptr(feats), _lib.ptr(out_feats), C,
-                                              _lib.ptr(in_to_out), _lib.ptr(seg_start), n, int(ctx.mode == "max"),
-                                              _lib.ptr(grad_in), _lib.stream_ptr()), "st_pool_bwd")
-        return grad_in, None, None, None, None, None, None, None
 
 
 def sparse_pooling(input: SparseTensor, kernel_size: int, padding: int, stride: int, mode: str) -> SparseTensor:

@@ -9,44 +9,19 @@ device->host read of `coords[:, 0].max()`; SparseTensor.dense() passes its own.
 """
 import torch
 
-from sparsetriton_b200 import _lib, trace
+from sparsetriton_b200 import _lib
 
 __all__ = ["to_dense", "ToDenseFunction"]
 
 
 class ToDenseFunction(torch.autograd.Function):
-    """feats (N, C), coords (N, 4) -> dense (batch, X, Y, Z, C); backward returns grad_feats only."""
+    """feats (N, C), coords (N, 4) -> dense (batch, X, Y, Z, C); backward gives grad_feats only.  `apply` makes the native
+    node (host/spatial.cpp)."""
 
     @staticmethod
-    def forward(ctx, feats, coords, spatial_range, batch_size):
+    def apply(feats, coords, spatial_range, batch_size):
         _lib.require_cuda(feats, "to_dense")
-        feats = feats.contiguous()
-        coords = coords.contiguous()
-        n, C = feats.shape
-        shape = tuple(int(v) for v in spatial_range)
-        dense = torch.empty((int(batch_size), *shape, C), dtype=feats.dtype, device=feats.device)
-        status = torch.zeros(1, dtype=torch.int32, device=feats.device)
-        with _lib.on_device(feats.device), trace.stage("to_dense_fwd"):
-            rc = _lib.lib().st_to_dense_fwd(_lib.feat_code(feats), _lib.ptr(feats), _lib.ptr(coords), _lib.coord_code(coords),
-                                            n, C, int(batch_size), _lib.host_i32(shape), _lib.ptr(dense), _lib.ptr(status),
-                                            _lib.stream_ptr())
-        _lib.check(rc, "st_to_dense_fwd")
-        ctx.save_for_backward(coords)
-        ctx.geometry = (n, C, int(batch_size), shape)
-        return dense
-
-    @staticmethod
-    def backward(ctx, grad_output):
-        (coords,) = ctx.saved_tensors
-        n, C, batch, shape = ctx.geometry
-        grad_output = grad_output.contiguous()
-        grad_feats = torch.empty((n, C), dtype=grad_output.dtype, device=grad_output.device)
-        with _lib.on_device(grad_output.device), trace.stage("to_dense_bwd"):
-            rc = _lib.lib().st_to_dense_bwd(_lib.feat_code(grad_output), _lib.ptr(grad_output), _lib.ptr(coords),
-                                            _lib.coord_code(coords), n, C, batch, _lib.host_i32(shape),
-                                            _lib.ptr(grad_feats), _lib.stream_ptr())
-        _lib.check(rc, "st_to_dense_bwd")
-        return grad_feats, None, None, None
+        return _lib.host().to_dense(feats, coords, [int(v) for v in spatial_range], int(batch_size))
 
 
 def to_dense(feats, coords, spatial_range, batch_size=None):

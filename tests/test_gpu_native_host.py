@@ -1,0 +1,161 @@
+"""The native host side and the kernels behind it at the sizes where they can go wrong: edges of tiles and rings, remainders,
+the smallest and largest of a range.  References are plain PyTorch in fp32, or the slower form of the same entry point."""
+import pytest
+import torch
+
+from sparsetriton_b200 import _lib, synthetic
+from sparsetriton_b200.config import get_coords_dtype, set_coords_dtype
+from sparsetriton_b200.nn.functional.conv.conv import compute_neighbor_indices
+from sparsetriton_b200.nn.functional.conv.kmap import build_out_coords
+from sparsetriton_b200.tensor import SparseTensor
+from sparsetriton_b200.utils.hash import HashTable
+
+pytestmark = pytest.mark.gpu
+TOL = {torch.float32: 2e-3, torch.bfloat16: 1e-2, torch.float16: 1e-2}
+
+
+def _rel(got, want):
+    got, want = got.double(), want.double()
+    return float((got - want).norm() / want.norm().clamp(min=1e-30))
+
+
+def _map(n_rows, n_src, K, density, seed):
+    g = torch.Generator().manual_seed(seed)
+    m = torch.randint(0, n_src, (n_rows, K), generator=g, dtype=torch.int32)
+    m[torch.rand(n_rows, K, generator=g) >= density] = -1
+    # at most one output per (input, offset), as in a convolution
+    for k in range(K):
+        seen = {}
+        col = m[:, k].tolist()
+        for o, i in enumerate(col):
+            if i >= 0 and i in seen:
+                m[o, k] = -1
+            seen[i] = o
+    return m
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16, torch.float32], ids=["bf16", "fp16", "fp32"])
+@pytest.mark.parametrize("n_rows,n_src,K,cin,cout,density", [
+    (1, 1, 1, 16, 16, 1.0), (127, 40, 27, 32, 64, 0.2), (128, 128, 8, 64, 32, 0.5), (129, 200, 27, 96, 48, 0.3),
+    (900, 700, 27, 256, 256, 0.4), (700, 900, 33, 48, 80, 0.1), (500, 500, 125, 128, 16, 0.05), (20000, 17000, 27, 64, 128, 0.15),
+    (300, 300, 27, 144, 240, 0.0)])
+def test_products_at_the_edges(cuda_device, dtype, n_rows, n_src, K, cin, cout, density):
+    H = _lib.host()
+    nbr = _map(n_rows, n_src, K, density, n_rows + K)
+    g = torch.Generator().manual_seed(cin)
+    x, w, dy = (torch.randn(s, generator=g).to(cuda_device, dtype) for s in ((n_src, cin), (K, cin, cout), (n_rows, cout)))
+    x.requires_grad_(True)
+    w.requires_grad_(True)
+    nbr = nbr.to(cuda_device)
+    y = H.conv(x, w, nbr, H.MapState(), True)
+    dx, dw = torch.autograd.grad(y, [x, w], dy)
+    torch.cuda.synchronize()
+    assert _lib.device_status(cuda_device)[0] == 0
+    xf, wf, dyf, have = x.detach().float(), w.detach().float(), dy.float(), nbr >= 0
+    want_y, want_dx, want_dw = torch.zeros(n_rows, cout, device=cuda_device), torch.zeros_like(xf), torch.zeros_like(wf)
+    for k in range(K):
+        o = have[:, k].nonzero()[:, 0]
+        i = nbr[o, k].long()
+        want_y[o] += xf[i] @ wf[k]
+        want_dx.index_add_(0, i, dyf[o] @ wf[k].t())
+        want_dw[k] = xf[i].t() @ dyf[o]
+    for got, want in ((y, want_y), (dx, want_dx), (dw, want_dw)):
+        assert got.dtype == dtype
+        assert _rel(got, want) < TOL[dtype] if want.abs().sum() > 0 else float(got.abs().sum()) == 0
+
+
+def test_fp32_weights_take_fp32_sums(cuda_device):
+    """16-bit features with fp32 master weights: dW arrives in fp32, unrounded."""
+    H = _lib.host()
+    nbr = _map(600, 500, 27, 0.3, 5).to(cuda_device)
+    x = torch.randn(500, 32, device=cuda_device).bfloat16()
+    w = torch.randn(27, 32, 64, device=cuda_device, requires_grad=True)
+    dy = torch.randn(600, 64, device=cuda_device).bfloat16()
+    (dw,) = torch.autograd.grad(H.conv(x, w, nbr, H.MapState(), True), [w], dy)
+    want = torch.zeros_like(w)
+    for k in range(27):
+        o = (nbr[:, k] >= 0).nonzero()[:, 0]
+        want[k] = x[nbr[o, k].long()].float().t() @ dy[o].float()
+    assert dw.dtype == torch.float32 and _rel(dw, want) < 1e-5
+
+
+@pytest.mark.parametrize("k,d,n,grid,dtype", [(3, 1, 230_000, 64, torch.int32), (3, 2, 230_000, 97, torch.int16),
+                                              (5, 1, 60_000, 40, torch.int32), (7, 1, 20_000, 33, torch.int32)])
+def test_map_by_columns_equals_full_probing(cuda_device, k, d, n, grid, dtype):
+    """From half a million probes on the symmetric map goes through the column filter; duplicates, negative cells and cells outside
+    the grid included."""
+    coords = synthetic.random_cells(n, 2, grid, seed=k)
+    coords[5] = coords[n // 2]
+    coords[7, 3] = -1
+    coords[9, 1] = grid + 40
+    coords = coords.to(cuda_device, dtype)
+    assert _lib.lib().st_map_build_symmetric_workspace_bytes(n, k ** 3) > 0
+    table = HashTable(1 << 20, device=cuda_device)
+    table.insert(coords)
+    _, _, off = build_out_coords(coords, (grid,) * 3, k, 1, d, (k - 1) * d // 2, submanifold=True)
+    want = compute_neighbor_indices(table, coords, off, (grid,) * 3, 1)
+    got = compute_neighbor_indices(table, coords, off, (grid,) * 3, 1, queries_are_table_rows=True)
+    assert torch.equal(got, want)
+
+
+@pytest.mark.parametrize("n", [1, 255, 1024, 1025, 700_001])
+@pytest.mark.parametrize("dtype", [torch.int16, torch.int32])
+def test_extent(cuda_device, n, dtype):
+    c = torch.randint(-500, 30_000, (n, 4), dtype=dtype, device=cuda_device)
+    for _ in range(3):                                        # the scratch has to be left as it was found
+        assert _lib.host().extent(c) == c.max(dim=0).values.tolist()
+
+
+@pytest.mark.parametrize("n,samples,order", [(1, 1, "sorted"), (2047, 3, "sorted"), (2049, 70, "mixed"), (300_000, 1500, "mixed")])
+def test_batch_info(cuda_device, n, samples, order):
+    b = torch.randint(-1, samples + 1, (n,), device=cuda_device)
+    b = b.sort().values if order == "sorted" else b
+    coords = torch.stack([b] + [torch.zeros_like(b)] * 3, 1).int()
+    ids, inv, status, first = _lib.host().batch_info(coords, samples)
+    ok = (b >= 0) & (b < samples)
+    counts = torch.bincount(b[ok], minlength=samples)
+    want_first = torch.full((samples,), n, device=cuda_device).scatter_reduce(0, b[ok], ok.nonzero()[:, 0], "amin")
+    assert torch.equal(ids.long(), b) and int(status) == 0
+    assert torch.equal(inv, 1.0 / counts.clamp(min=1).float())
+    assert torch.equal(first.long(), torch.where(counts > 0, want_first, -1))
+
+
+@pytest.mark.parametrize("C", [8, 20, 64])
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32], ids=["bf16", "fp32"])
+def test_batch_norm_over_running_statistics(cuda_device, C, dtype):
+    g = torch.Generator().manual_seed(C)
+    x, w, b, m = (torch.randn(s, generator=g).to(cuda_device) for s in ((333, C), (C,), (C,), (C,)))
+    v = torch.rand(C, generator=g).to(cuda_device) + 0.1
+    x = x.to(dtype).requires_grad_(True)
+    w.requires_grad_(True)
+    y = _lib.host().batch_norm_running(x, w, b, m, v, 1e-5, True)
+    xr = x.detach().float().requires_grad_(True)
+    wr = w.detach().clone().requires_grad_(True)
+    want = torch.relu((xr - m) * torch.rsqrt(v + 1e-5) * wr + b)
+    dy = torch.randn_like(want).to(dtype)
+    got_g, want_g = torch.autograd.grad(y, [x, w], dy), torch.autograd.grad(want, [xr, wr], dy.float())
+    for a, c in zip((y,) + got_g, (want,) + want_g):
+        assert _rel(a, c) < (1e-5 if dtype == torch.float32 else 1e-2)
+
+
+@pytest.mark.parametrize("mode", ["max", "avg"])
+@pytest.mark.parametrize("C", [5, 8, 64])
+@pytest.mark.parametrize("grid,n", [(9, 300), (40, 30_000)])
+def test_pooling_forward_and_gradient(cuda_device, mode, C, grid, n):
+    """Whole 16-byte rows (C = 8, 64) and others (C = 5) against a reduction by cell."""
+    from sparsetriton_b200.nn.functional.spatial import sparse_pooling
+    before = get_coords_dtype()
+    set_coords_dtype(torch.int32)
+    try:
+        c = synthetic.random_cells(n, 2, grid, seed=n).to(cuda_device)
+        x = torch.randn(n, C, device=cuda_device, requires_grad=True)
+        out = sparse_pooling(SparseTensor(x, c, (grid,) * 3, 2), 4, 2, 4, mode)
+        key = ((c[:, 0].long() * 64 + c[:, 1] // 4) * 64 + c[:, 2] // 4) * 64 + c[:, 3] // 4
+        cells, inv = torch.unique(key, return_inverse=True)
+        want = torch.zeros(cells.shape[0], C, device=cuda_device).scatter_reduce(
+            0, inv[:, None].expand(-1, C), x, "amax" if mode == "max" else "mean", include_self=False)
+        dy = torch.randn_like(want)
+        assert torch.allclose(out.F, want, atol=1e-6)
+        assert torch.allclose(torch.autograd.grad(out.F, x, dy)[0], torch.autograd.grad(want, x, dy)[0], atol=1e-6)
+    finally:
+        set_coords_dtype(before)
