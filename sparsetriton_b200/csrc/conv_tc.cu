@@ -43,6 +43,17 @@ constexpr int kGatherThreads = (kEpilogueWarps + 1 + kGatherGroups * kProducerWa
 constexpr int kABlockBytes = kTileM * 128;                     // 128 rows x 128 B
 
 
+// Two fp32 accumulators as a pair of 16-bit outputs.
+__device__ __forceinline__ uint32_t pack_pair(int out_kind, uint32_t a, uint32_t b) {
+  const float lo = __uint_as_float(a), hi = __uint_as_float(b);
+  if (out_kind == ST_BF16) {
+    __nv_bfloat162 h = __floats2bfloat162_rn(lo, hi);
+    return *reinterpret_cast<uint32_t*>(&h);
+  }
+  __half2 h = __floats2half2_rn(lo, hi);
+  return *reinterpret_cast<uint32_t*>(&h);
+}
+
 // Store 32 fp32 accumulator columns of one row.
 template <int N>
 __device__ __forceinline__ void store_cols(void* out_row, int col0, int out_kind, const uint32_t* v) {
@@ -58,16 +69,7 @@ __device__ __forceinline__ void store_cols(void* out_row, int col0, int out_kind
     for (int i = 0; i < N / 8; ++i) {
       uint32_t p[4];
 #pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        float lo = __uint_as_float(v[8 * i + 2 * j]), hi = __uint_as_float(v[8 * i + 2 * j + 1]);
-        if (out_kind == ST_BF16) {
-          __nv_bfloat162 h = __floats2bfloat162_rn(lo, hi);
-          p[j] = *reinterpret_cast<uint32_t*>(&h);
-        } else {
-          __half2 h = __floats2half2_rn(lo, hi);
-          p[j] = *reinterpret_cast<uint32_t*>(&h);
-        }
-      }
+      for (int j = 0; j < 4; ++j) p[j] = pack_pair(out_kind, v[8 * i + 2 * j], v[8 * i + 2 * j + 1]);
       dst[i] = make_uint4(p[0], p[1], p[2], p[3]);
     }
   }
@@ -1171,7 +1173,7 @@ static bool fill_params2(tc::Params2* p, int dtype, const void* in, const void* 
   p->w_slots = 3;
   p->idx_bytes = planned ? 0 : tc::kIdxTileBytes;
   p->w_flip = 0;
-  const int budget = 222 * 1024 - p->idx_bytes;
+  const int budget = 224 * 1024 - (planned ? 4 * (int)tc::kOutWarpBytes : 2048 + p->idx_bytes);
   int a_stages = (budget - p->w_slots * p->w_slot_bytes) / tc::kABlockBytes;
   if (a_stages > tc::kMaxAStages) a_stages = tc::kMaxAStages;
   if (a_stages < 4) {
@@ -1302,7 +1304,8 @@ static int launch_planned(tc::Params2 p, const tc::PlannedRows& map, cudaStream_
                        make_weight_desc(&w_desc, p.w, (int64_t)p.K * p.w_rows, p.w_cols, p.esize, p.out_kind,
                                         p.b_mn_major ? 128 / p.esize : p.w_rows, p.b_mn_major && p.esize == 4);
   if (!planned) return launch_gather(p, map, stream);
-  const size_t smem = (size_t)p.w_slots * p.w_slot_bytes + (size_t)p.a_stages * tc::kABlockBytes + sizeof(tc::Control3) + 1024;
+  const size_t smem = (size_t)p.w_slots * p.w_slot_bytes + (size_t)p.a_stages * tc::kABlockBytes + 4 * tc::kOutWarpBytes +
+                      sizeof(tc::Control3) + 1024;
   auto kernel = p.esize == 2 ? tc::planned_gather_kernel<2> : tc::planned_gather_kernel<4>;
   static bool configured[kMaxDevices] = {};
   if (!configured[current_device()]) {

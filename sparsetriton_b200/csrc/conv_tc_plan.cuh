@@ -20,7 +20,7 @@
 //
 // Hand-over of a stage: 128 arrivals would serialise on its mbarrier, so a warp closes its share of a stage with
 // cp.async.commit_group and arrives for it (one lane) when its next share is on its way.  (Two shares on their way: up to
-// 6 % slower, a stage then waits for one eight stages behind it.)  The warp that issues the MMAs fences the proxies.
+// 6 % slower, a stage then waits for one eight stages behind it.)
 #pragma once
 
 namespace st {
@@ -118,6 +118,52 @@ __device__ __forceinline__ void fetch_block(uint32_t dst, int row0, int idx, con
   else fetch_rows<1, kRows, kAtom32>(dst, row0, idx, col, pitch, n_src, chunks, lane);
 }
 
+// Accumulator columns c0 .. of a warp's 32 rows (lane = row) to the output rows `dst` (-1: none), P 16-byte pieces of each,
+// by way of shared memory: there a lane has a row, in the stores P lanes share one.  With lane = row in the stores as well
+// (16 bytes of 32 rows per instruction) the accumulators took as long to drain as to fill: 60 of 227 us at 815249 rows of 64 -> 128.
+constexpr uint32_t kOutWarpBytes = 32 * 128;
+template <int P>
+__device__ __forceinline__ void store_block(const Params2& p, uint32_t stage, uint32_t t_row, int c0, int dst, bool zeros, int lane) {
+  constexpr int kRowsPerLine = 8 / P;                         // rows of 128 bytes, pieces swizzled within
+  auto at = [&](int row, int piece) {
+    return stage + (uint32_t)(row / kRowsPerLine) * 128u +
+           (uint32_t)((row & (kRowsPerLine - 1)) * P + (piece ^ ((row / kRowsPerLine) & (P - 1)))) * 16u;
+  };
+  auto put = [&](int piece, const uint32_t* w) {
+    asm volatile("st.shared.v4.b32 [%0], {%1,%2,%3,%4};" ::"r"(at(lane, piece)), "r"(zeros ? 0u : w[0]), "r"(zeros ? 0u : w[1]),
+                 "r"(zeros ? 0u : w[2]), "r"(zeros ? 0u : w[3]) : "memory");
+  };
+  const bool f32 = p.out_kind == ST_F32;
+  const int es = f32 ? 4 : 2, cols = P * 16 / es;
+  for (int c = 0; c < cols; c += 16) {
+    uint32_t v[32];                                            // 16 are used
+    tmem_ld16(t_row + (uint32_t)(c0 + c), v);
+    tmem_ld_wait();
+    if (f32) {
+#pragma unroll
+      for (int i = 0; i < 4; ++i) put(c / 4 + i, v + 4 * i);
+    } else {
+      uint32_t w[8];
+#pragma unroll
+      for (int i = 0; i < 8; ++i) w[i] = pack_pair(p.out_kind, v[2 * i], v[2 * i + 1]);
+      put(c / 8, w);
+      put(c / 8 + 1, w + 4);
+    }
+  }
+  __syncwarp();
+  char* out = static_cast<char*>(p.out) + (size_t)c0 * es + (lane % P) * 16;
+  const size_t pitch = (size_t)p.c_acc * es;
+#pragma unroll
+  for (int i = 0; i < P; ++i) {
+    const int row = i * (32 / P) + lane / P;
+    const int to = __shfl_sync(0xFFFFFFFFu, dst, row);
+    uint4 v;
+    asm volatile("ld.shared.v4.b32 {%0,%1,%2,%3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(at(row, lane % P)) : "memory");
+    if (to >= 0) *reinterpret_cast<uint4*>(out + (size_t)to * pitch) = v;
+  }
+  __syncwarp();
+}
+
 template <int ESIZE>
 __global__ void __launch_bounds__(kGather3Threads, 1) planned_gather_kernel(const Params2 p, const PlannedRows map,
                                                                             const __grid_constant__ CUtensorMap w_desc) {
@@ -126,7 +172,8 @@ __global__ void __launch_bounds__(kGather3Threads, 1) planned_gather_kernel(cons
   const uint32_t base = (raw + 1023u) & ~1023u;
   unsigned char* base_ptr = smem_raw + (base - raw);
   const uint32_t a_ring = base + (uint32_t)p.w_slots * (uint32_t)p.w_slot_bytes;
-  Control3* ctl = reinterpret_cast<Control3*>(base_ptr + (size_t)p.w_slots * p.w_slot_bytes + (size_t)p.a_stages * kABlockBytes);
+  const uint32_t out_ring = a_ring + (uint32_t)p.a_stages * kABlockBytes;
+  Control3* ctl = reinterpret_cast<Control3*>(base_ptr + (out_ring - base) + 4 * kOutWarpBytes);
   volatile int* abort_flag = &ctl->abort_flag;
   const int warp = __shfl_sync(0xFFFFFFFFu, (int)(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;
 
@@ -178,6 +225,7 @@ __global__ void __launch_bounds__(kGather3Threads, 1) planned_gather_kernel(cons
                          min(128, red_bytes - pend_kb * 128), lane);
       cp_async_commit();
       cp_async_wait_group<1>();                               // the share before this one has landed: announce it
+      fence_proxy_async();
       __syncwarp();
       if (sent >= 0 && lane == 0) mbar_arrive(smem_u32(&ctl->a_full[sent]));
       sent = pend_stage;
@@ -208,6 +256,7 @@ __global__ void __launch_bounds__(kGather3Threads, 1) planned_gather_kernel(cons
     }, nothing);
     if (pend_stage >= 0 && ok) run();
     cp_async_wait_all();
+    fence_proxy_async();
     __syncwarp();
     if (sent >= 0 && lane == 0) mbar_arrive(smem_u32(&ctl->a_full[sent]));
   } else if (warp == kWarpW) {
@@ -255,6 +304,7 @@ __global__ void __launch_bounds__(kGather3Threads, 1) planned_gather_kernel(cons
     {
       int stage = 0, slot = 0;
       uint32_t phase = 0, w_phase = 0;
+      bool a_ready = false, w_ready = false;                   // what a look ahead at the next stage and slot said
       uint32_t acc_phase[2] = {0, 0};
       int buf = 0;
       const uint32_t b_kstep16 = (p.b_mn_major ? (32 / ESIZE) * 128 : 32) >> 4;   // K-step advance, 16-byte units
@@ -270,16 +320,21 @@ __global__ void __launch_bounds__(kGather3Threads, 1) planned_gather_kernel(cons
           return ok;
         },
         [&](int64_t, int, int kb, uint32_t users, uint32_t fresh) {
-          if (!mbar_wait_all(smem_u32(&ctl->w_full[slot]), w_phase, abort_flag, 33)) return false;
+          if (!__all_sync(0xFFFFFFFFu, w_ready) && !mbar_wait_all(smem_u32(&ctl->w_full[slot]), w_phase, abort_flag, 33)) return false;
           const uint32_t w_lo = (base + (uint32_t)slot * (uint32_t)p.w_slot_bytes) >> 4;
           const int ksteps = min(128, red_bytes - kb * 128) >> 5;
 #pragma unroll
           for (int s = 0; s < kMaxSub; ++s) {
             if (!((users >> s) & 1u)) continue;
-            if (!mbar_wait_all(smem_u32(&ctl->a_full[stage]), phase, abort_flag, 34)) return false;
-            fence_proxy_async();                                                 // rows were written by cp.async
+            if (!__all_sync(0xFFFFFFFFu, a_ready) && !mbar_wait_all(smem_u32(&ctl->a_full[stage]), phase, abort_flag, 34)) return false;
+            const int this_stage = stage;
+            if (++stage == p.a_stages) {
+              stage = 0;
+              phase ^= 1u;
+            }
+            a_ready = mbar_try_now(smem_u32(&ctl->a_full[stage]), phase);
             tc_fence_after();
-            const uint32_t a_lo = (a_ring + (uint32_t)stage * kABlockBytes) >> 4;
+            const uint32_t a_lo = (a_ring + (uint32_t)this_stage * kABlockBytes) >> 4;
             const uint32_t d_addr = tmem_base + (uint32_t)(buf * set_cols + s * p.c_acc);
             const uint32_t add = ((fresh >> s) & 1u) ? 0u : 1u;                  // 0: the first MMA overwrites
             if (elect_one()) {
@@ -294,11 +349,7 @@ __global__ void __launch_bounds__(kGather3Threads, 1) planned_gather_kernel(cons
                     mma_tf32(d_addr, da, db, idesc, ks == 0 ? add : 1u);
                 }
               }
-              mma_commit(smem_u32(&ctl->a_empty[stage]));
-            }
-            if (++stage == p.a_stages) {
-              stage = 0;
-              phase ^= 1u;
+              mma_commit(smem_u32(&ctl->a_empty[this_stage]));
             }
           }
           if (elect_one()) mma_commit(smem_u32(&ctl->w_empty[slot]));
@@ -306,6 +357,7 @@ __global__ void __launch_bounds__(kGather3Threads, 1) planned_gather_kernel(cons
             slot = 0;
             w_phase ^= 1u;
           }
+          w_ready = mbar_try_now(smem_u32(&ctl->w_full[slot]), w_phase);
           return true;
         },
         [&](int64_t) {
@@ -322,10 +374,7 @@ __global__ void __launch_bounds__(kGather3Threads, 1) planned_gather_kernel(cons
     int buf = 0;
     bool ok = true;
     const int out_es = p.out_kind == ST_F32 ? 4 : 2;
-    auto zero = [](uint32_t (&v)[32]) {
-#pragma unroll
-      for (int i = 0; i < 32; ++i) v[i] = 0u;
-    };
+    const uint32_t stage_rows = out_ring + (uint32_t)warp * kOutWarpBytes;
     for (int64_t st_i = blockIdx.x; st_i < p.n_super && ok; st_i += gridDim.x) {
       // where this lane's rows go: known before the accumulators are ready, so fetched before the wait
       int64_t dst_rows[kMaxSub];
@@ -349,22 +398,16 @@ __global__ void __launch_bounds__(kGather3Threads, 1) planned_gather_kernel(cons
         if (s >= p.sub) break;
         const int64_t row = (st_i * p.sub + s) * (int64_t)kTileM + warp * 32 + lane;
         if ((st_i * p.sub + s) * (int64_t)kTileM >= p.n_rows) break;         // whole sub tile past the end
-        char* out_row = static_cast<char*>(p.out) + (size_t)dst_rows[s] * p.c_acc * out_es;
         const uint32_t t_row = tmem_base + ((uint32_t)(warp * 32) << 16) + (uint32_t)(buf * set_cols + s * p.c_acc);
-        for (int c0 = 0; c0 < p.c_acc; c0 += 32) {
-          uint32_t v[32];
-          if (p.c_acc - c0 >= 32) {
-            tmem_ld32(t_row + c0, v);
-            tmem_ld_wait();
-            if (!((touched >> s) & 1u)) zero(v);
-            if (row < p.n_rows) store_cols<32>(out_row, c0, p.out_kind, v);
-          } else {
-            tmem_ld16(t_row + c0, v);
-            tmem_ld_wait();
-            if (!((touched >> s) & 1u)) zero(v);
-            if (row < p.n_rows) store_cols<16>(out_row, c0, p.out_kind, v);
-          }
+        const int dst = row < p.n_rows ? (int)dst_rows[s] : -1;
+        const bool zeros = !((touched >> s) & 1u);
+        int c0 = 0;
+        for (; p.c_acc - c0 >= 128 / out_es; c0 += 128 / out_es) store_block<8>(p, stage_rows, t_row, c0, dst, zeros, lane);
+        if (p.c_acc - c0 >= 64 / out_es) {
+          store_block<4>(p, stage_rows, t_row, c0, dst, zeros, lane);
+          c0 += 64 / out_es;
         }
+        if (c0 < p.c_acc) store_block<2>(p, stage_rows, t_row, c0, dst, zeros, lane);
       }
       tc_fence_before();
       mbar_arrive(smem_u32(&ctl->acc_empty[buf]));
