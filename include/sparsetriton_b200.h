@@ -240,6 +240,14 @@ int st_conv_dgrad(int dtype, const void* dY, const void* W, const int32_t* inv, 
 int st_conv_wgrad(int dtype, const void* X, const void* dY, const int32_t* nbr, void* dW, int64_t n_in,
                   int64_t n_out, int K, int cin, int cout, void* workspace, int64_t workspace_bytes, void* stream);
 
+/* st_map_plan(sort_rows = 1) and st_map_plan_inverse for K <= 32 with whole tiles of 128 rows moved: most offsets first, equal
+ * numbers in mask order, a tile that is not full last.  Only the lines of tmap whose bit is set in tmask are written. */
+int64_t st_map_plan_balanced_workspace_bytes(int64_t n_rows, int K);
+int st_map_plan_balanced(const int32_t* nbr, int64_t n_rows, int K, int32_t* order, int32_t* tmap, uint32_t* tmask,
+                         void* workspace, int64_t workspace_bytes, void* stream);
+int st_map_plan_inverse_balanced(const int32_t* nbr, int64_t n_out, int K, int64_t n_in, int32_t* order, int32_t* tmap,
+                                 uint32_t* tmask, void* workspace, int64_t workspace_bytes, void* stream);
+
 /* The three products over a map that comes with a tile plan from st_map_plan() (of the map they are
  * given: the forward map for fwd and wgrad, the inverse map for dgrad).  row_order, tmap and tmask
  * may each be NULL: without tmap/tmask the kernels read `nbr` itself, without row_order they walk

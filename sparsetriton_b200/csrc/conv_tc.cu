@@ -1318,8 +1318,7 @@ static int launch_planned(tc::Params2 p, const tc::PlannedRows& map, cudaStream_
     }
     configured[current_device()] = true;
   }
-  const int64_t grid = p.n_super < sm_count() ? p.n_super : sm_count();
-  kernel<<<(unsigned)grid, tc::kGather3Threads, smem, stream>>>(p, map, w_desc);
+  kernel<<<(unsigned)p.n_super, tc::kGather3Threads, smem, stream>>>(p, map, w_desc);
   note_launches(1);
   return check_launch("tc planned gather");
 }

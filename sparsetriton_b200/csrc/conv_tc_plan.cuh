@@ -8,8 +8,12 @@
 // each sub tile that has the offset sends one stage of 128 gathered rows through the ring of row stages.
 //
 // Warps 0-3 drain accumulators, warp 4 issues the MMAs, warp 5 fetches W slices by TMA, warps 6-21 fetch rows with
-// 16-byte cp.async: four groups of four warps take the stages in turn, a warp has 32 rows of a stage.  All of them walk
-// the tile masks themselves, so nothing but data and barriers goes through shared memory.
+// 16-byte cp.async: four groups of four warps take the stages in turn, a warp has 32 rows of a stage.  Warp 22 hands out
+// super tiles with their tile masks, which the others walk themselves.
+//
+// Who does which super tile: super tiles cost 1 to K offsets, and dealt out in a fixed pattern the busiest SM had 1.3 to 2
+// times the mean.  The grid is one CTA per super tile, and a CTA that runs takes over others before they start
+// (clusterlaunchcontrol); plans of sorted rows put their tiles in descending order of work, so the last ones are small.
 //
 // What bounds it: bringing rows into shared memory.  A loop that does nothing else (148 CTAs, random rows) takes, per
 // stage of 128 rows, with tile::gather4 612-743 cycles when every row exists and 1180 (128-byte rows) to 1880
@@ -29,47 +33,72 @@ namespace tc {
 constexpr int kRowGroups = 4, kRowGroupWarps = 4;             // warps that fetch rows
 constexpr int kWarpW = kMmaWarp + 1;                          // the warp that fetches W slices
 constexpr int kFirstRowWarp = kWarpW + 1;
-constexpr int kGather3Threads = (kFirstRowWarp + kRowGroups * kRowGroupWarps) * 32;
+constexpr int kWarpJobs = kFirstRowWarp + kRowGroups * kRowGroupWarps;
+constexpr int kGather3Threads = (kWarpJobs + 1) * 32;
+constexpr int kJobReaders = kWarpJobs;                        // all warps before it
+// Super tiles on offer at a time.  Every one taken early is one that cannot go to an SM that turns out to be free.
+constexpr int kJobs = 2;
+
+struct Job {
+  int super;                                                   // -1: no more
+  uint32_t touched;                                            // its sub tiles that have any offset
+  uint32_t mask[kMaxSub];                                      // offsets 0 .. 31
+};
 
 struct __align__(8) Control3 {
   unsigned long long a_full[kMaxAStages], a_empty[kMaxAStages];
   unsigned long long w_full[kMaxWSlots], w_empty[kMaxWSlots];
   unsigned long long acc_full[2], acc_empty[2];
+  unsigned long long job_full[kJobs], job_empty[kJobs], taken;
+  __align__(16) uint4 taken_cta;
+  Job job[kJobs];
   uint32_t tmem_base;
   int abort_flag;
+};
+
+// A warp's view of the super tiles this CTA has, in order.
+struct JobReader {
+  Control3* ctl;
+  volatile int* abort_flag;
+  int lane;
+  int slot = 0;
+  uint32_t phase = 0;
+  Job job;
+  // before_wait(): what others may need from this warp before the next job can come.
+  template <typename F>
+  __device__ __forceinline__ bool next(F&& before_wait) {
+    if (!__all_sync(0xFFFFFFFFu, mbar_try_now(smem_u32(&ctl->job_full[slot]), phase))) before_wait();
+    if (!mbar_wait_all(smem_u32(&ctl->job_full[slot]), phase, abort_flag, 43)) return false;
+    job = ctl->job[slot];
+    __syncwarp();
+    if (lane == 0) mbar_arrive(smem_u32(&ctl->job_empty[slot]));
+    if (++slot == kJobs) {
+      slot = 0;
+      phase ^= 1u;
+    }
+    return __all_sync(0xFFFFFFFFu, job.super >= 0);
+  }
 };
 
 // The work of this CTA in order: item(tile0, k, kb, users, fresh) for every occupied (offset, 128-byte block) of a
 // super tile (users: the sub tiles that have the offset; fresh: those whose accumulator starts here), between
 // begin(tile0) and end(tile0).  Stops when one of them returns false.
-template <typename Begin, typename Item, typename End>
-__device__ __forceinline__ void walk_super_tiles(const Params2& p, const PlannedRows& map, int64_t n_tiles, Begin&& begin,
-                                                 Item&& item, End&& end) {
-  auto load_masks = [&](int64_t tile0, int word, uint32_t* m) {
-#pragma unroll
-    for (int s = 0; s < kMaxSub; ++s)
-      m[s] = (s < p.sub && tile0 + s < n_tiles) ? __ldg(map.tmask + (tile0 + s) * map.MW + word) : 0u;
-  };
-  // every lane loads the same words; the reduction tells the compiler so (uniform registers and branches)
-  auto uniform = [](uint32_t* m) {
-#pragma unroll
-    for (int s = 0; s < kMaxSub; ++s) m[s] = __reduce_or_sync(0xFFFFFFFFu, m[s]);
-  };
-  uint32_t next_m[kMaxSub];
-  load_masks((int64_t)blockIdx.x * p.sub, 0, next_m);
-  for (int64_t st_i = blockIdx.x; st_i < p.n_super; st_i += gridDim.x) {
-    const int64_t tile0 = st_i * p.sub;
+template <typename Idle, typename Begin, typename Item, typename End>
+__device__ __forceinline__ void walk_super_tiles(const Params2& p, const PlannedRows& map, int64_t n_tiles, JobReader jobs,
+                                                 Idle&& before_wait, Begin&& begin, Item&& item, End&& end) {
+  while (jobs.next(before_wait)) {
+    const int64_t tile0 = (int64_t)jobs.job.super * p.sub;
+    // every lane has the same words; the reduction tells the compiler so (uniform registers and branches)
     uint32_t m[kMaxSub];
 #pragma unroll
-    for (int s = 0; s < kMaxSub; ++s) m[s] = next_m[s];
-    uniform(m);
-    if (st_i + gridDim.x < p.n_super) load_masks((st_i + gridDim.x) * p.sub, 0, next_m);
+    for (int s = 0; s < kMaxSub; ++s) m[s] = __reduce_or_sync(0xFFFFFFFFu, jobs.job.mask[s]);
     if (!begin(tile0)) return;
     uint32_t touched = 0;
     for (int word = 0; word < map.MW; ++word) {
       if (word) {
-        load_masks(tile0, word, m);
-        uniform(m);
+#pragma unroll
+        for (int s = 0; s < kMaxSub; ++s)
+          m[s] = __reduce_or_sync(0xFFFFFFFFu, s < p.sub && tile0 + s < n_tiles ? __ldg(map.tmask + (tile0 + s) * map.MW + word) : 0u);
       }
       static_assert(kMaxSub == 4, "the masks of a super tile are combined by hand");
       uint32_t m_any = m[0] | m[1] | m[2] | m[3];
@@ -190,6 +219,11 @@ __global__ void __launch_bounds__(kGather3Threads, 1) planned_gather_kernel(cons
       mbar_init(smem_u32(&ctl->acc_full[b]), 1);
       mbar_init(smem_u32(&ctl->acc_empty[b]), kEpilogueWarps * 32);
     }
+    for (int s = 0; s < kJobs; ++s) {
+      mbar_init(smem_u32(&ctl->job_full[s]), 1);
+      mbar_init(smem_u32(&ctl->job_empty[s]), kJobReaders);
+    }
+    mbar_init(smem_u32(&ctl->taken), 1);
     ctl->abort_flag = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
@@ -205,8 +239,57 @@ __global__ void __launch_bounds__(kGather3Threads, 1) planned_gather_kernel(cons
   const int set_cols = p.sub * p.c_acc;                      // TMEM columns of one accumulator set
   const int64_t n_tiles = (p.n_rows + kTileM - 1) / kTileM;
   auto nothing = [](int64_t) { return true; };
+  const JobReader jobs{ctl, abort_flag, lane};
 
-  if (warp >= kFirstRowWarp) {
+  if (warp == kWarpJobs) {
+    // =============================================================== super tiles
+    int super = blockIdx.x, slot = 0;
+    uint32_t phase = 0, taken_phase = 0;
+    while (true) {
+      if (!mbar_wait_all(smem_u32(&ctl->job_empty[slot]), phase ^ 1u, abort_flag, 41)) break;
+      if (super < 0) {                                         // not the first: take over a CTA that has not started
+        if (lane == 0) {
+          mbar_arrive_expect_tx(smem_u32(&ctl->taken), 16);
+          take_cta(smem_u32(&ctl->taken_cta), smem_u32(&ctl->taken));
+        }
+        __syncwarp();
+        if (!mbar_wait_all(smem_u32(&ctl->taken), taken_phase, abort_flag, 42)) break;
+        taken_phase ^= 1u;
+        super = taken_cta(smem_u32(&ctl->taken_cta));
+        fence_proxy_async();                                   // read before the next answer is written
+      }
+      // masks of the first 32 offsets by lane = sub tile; all words for "has any"
+      uint32_t mask = 0, any = 0;
+      const int64_t tile = (int64_t)super * p.sub + lane;
+      if (super >= 0 && lane < p.sub && tile < n_tiles) {
+        mask = any = __ldg(map.tmask + tile * map.MW);
+        for (int word = 1; word < map.MW; ++word) any |= __ldg(map.tmask + tile * map.MW + word);
+      }
+      const uint32_t touched = __ballot_sync(0xFFFFFFFFu, any != 0u);
+      if (lane < kMaxSub) ctl->job[slot].mask[lane] = mask;
+      if (lane == 0) {
+        ctl->job[slot].super = super;
+        ctl->job[slot].touched = touched;
+      }
+      __syncwarp();
+      if (lane == 0) mbar_arrive(smem_u32(&ctl->job_full[slot]));
+      if (super < 0) break;
+      // its index lines: have them in L2 by the time the row warps ask
+      for (int s = 0; s < p.sub; ++s) {
+        const uint32_t m = __shfl_sync(0xFFFFFFFFu, mask, s);
+        if ((m >> lane) & 1u) {
+          const char* line = reinterpret_cast<const char*>(map.tmap + (((int64_t)super * p.sub + s) * map.K + lane) * kTileM);
+#pragma unroll
+          for (int i = 0; i < 4; ++i) prefetch_l2(line + i * 128);
+        }
+      }
+      super = -1;
+      if (++slot == kJobs) {
+        slot = 0;
+        phase ^= 1u;
+      }
+    }
+  } else if (warp >= kFirstRowWarp) {
     // =============================================================== rows
     static_assert(kRowGroups == kMaxSub, "an offset has at most one stage per group");
     const int group = (warp - kFirstRowWarp) / kRowGroupWarps;
@@ -230,7 +313,17 @@ __global__ void __launch_bounds__(kGather3Threads, 1) planned_gather_kernel(cons
       if (sent >= 0 && lane == 0) mbar_arrive(smem_u32(&ctl->a_full[sent]));
       sent = pend_stage;
     };
-    walk_super_tiles(p, map, n_tiles, nothing, [&](int64_t tile0, int k, int kb, uint32_t users, uint32_t) {
+    auto flush = [&]() {
+      // the job that this warp is about to wait for may wait for the stages that it has not announced
+      if (pend_stage >= 0 && ok) run();
+      pend_stage = -1;
+      cp_async_wait_all();
+      fence_proxy_async();
+      __syncwarp();
+      if (sent >= 0 && lane == 0) mbar_arrive(smem_u32(&ctl->a_full[sent]));
+      sent = -1;
+    };
+    walk_super_tiles(p, map, n_tiles, jobs, flush, nothing, [&](int64_t tile0, int k, int kb, uint32_t users, uint32_t) {
       const int n = __popc(users), mine = (group - turn) & (kRowGroups - 1);
       if (mine < n) {
         // this stage's row numbers are loaded now and its copies issued when the group's next stage comes up, so that
@@ -254,11 +347,7 @@ __global__ void __launch_bounds__(kGather3Threads, 1) planned_gather_kernel(cons
       }
       return ok;
     }, nothing);
-    if (pend_stage >= 0 && ok) run();
-    cp_async_wait_all();
-    fence_proxy_async();
-    __syncwarp();
-    if (sent >= 0 && lane == 0) mbar_arrive(smem_u32(&ctl->a_full[sent]));
+    flush();
   } else if (warp == kWarpW) {
     // =============================================================== W slices
     const int w_col_bytes = p.w_cols * ESIZE;
@@ -266,15 +355,7 @@ __global__ void __launch_bounds__(kGather3Threads, 1) planned_gather_kernel(cons
     const uint32_t w_bytes = p.b_mn_major ? (uint32_t)(((w_col_bytes + 127) >> 7) * kr * 128) : (uint32_t)(p.w_rows * 128);
     int slot = 0;
     uint32_t phase = 0;
-    auto prefetch = [&](int64_t tile0) {
-      // the index lines of a super tile are one contiguous block of the plan: have the next one in L2
-      const int64_t next_tile0 = tile0 + (int64_t)gridDim.x * p.sub;
-      const int64_t lines = min(min((int64_t)p.sub, n_tiles - next_tile0) * map.K * 4, (int64_t)1024);   // of 128 bytes
-      const char* block = reinterpret_cast<const char*>(map.tmap + next_tile0 * map.K * (int64_t)kTileM);
-      for (int64_t l = lane; l < lines; l += 32) prefetch_l2(block + l * 128);
-      return true;
-    };
-    walk_super_tiles(p, map, n_tiles, prefetch, [&](int64_t, int k, int kb, uint32_t, uint32_t) {
+    walk_super_tiles(p, map, n_tiles, jobs, [] {}, nothing, [&](int64_t, int k, int kb, uint32_t, uint32_t) {
       if (!mbar_wait_all(smem_u32(&ctl->w_empty[slot]), phase ^ 1u, abort_flag, 35)) return false;
       if (lane == 0) {
         const uint32_t bar = smem_u32(&ctl->w_full[slot]);
@@ -313,7 +394,7 @@ __global__ void __launch_bounds__(kGather3Threads, 1) planned_gather_kernel(cons
       const uint64_t a_desc_hi = smem_desc(0u, 16u, 1024u, 2u);
       const uint64_t b_desc_hi = smem_desc(0u, b_lbo, b_base32 ? 512u : 1024u, b_base32 ? 1u : 2u);
       const uint32_t idesc = p.idesc;
-      walk_super_tiles(p, map, n_tiles,
+      walk_super_tiles(p, map, n_tiles, jobs, [] {},
         [&](int64_t) {
           const bool ok = mbar_wait_all(smem_u32(&ctl->acc_empty[buf]), acc_phase[buf] ^ 1u, abort_flag, 32);
           tc_fence_after();
@@ -375,7 +456,9 @@ __global__ void __launch_bounds__(kGather3Threads, 1) planned_gather_kernel(cons
     bool ok = true;
     const int out_es = p.out_kind == ST_F32 ? 4 : 2;
     const uint32_t stage_rows = out_ring + (uint32_t)warp * kOutWarpBytes;
-    for (int64_t st_i = blockIdx.x; st_i < p.n_super && ok; st_i += gridDim.x) {
+    JobReader mine = jobs;
+    while (ok && mine.next([] {})) {
+      const int64_t st_i = mine.job.super;
       // where this lane's rows go: known before the accumulators are ready, so fetched before the wait
       int64_t dst_rows[kMaxSub];
 #pragma unroll
@@ -383,12 +466,7 @@ __global__ void __launch_bounds__(kGather3Threads, 1) planned_gather_kernel(cons
         const int64_t row = (st_i * p.sub + s) * (int64_t)kTileM + warp * 32 + lane;
         dst_rows[s] = (s < p.sub && p.order && row < p.n_rows) ? (int64_t)__ldg(p.order + row) : row;
       }
-      // sub tiles without any neighbour have no accumulator: their rows are zeros
-      uint32_t touched = 0;
-#pragma unroll
-      for (int s = 0; s < kMaxSub; ++s)
-        for (int word = 0; word < map.MW; ++word)
-          if (s < p.sub && st_i * p.sub + s < n_tiles && __ldg(map.tmask + (st_i * p.sub + s) * map.MW + word)) touched |= 1u << s;
+      const uint32_t touched = mine.job.touched;               // the others have no accumulator: their rows are zeros
       ok = mbar_wait(smem_u32(&ctl->acc_full[buf]), acc_phase[buf], abort_flag, 40, 256);
       ok = __all_sync(0xFFFFFFFFu, ok);
       if (!ok) break;

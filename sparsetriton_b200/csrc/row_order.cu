@@ -20,8 +20,10 @@ namespace {
 // key[r] = occupancy mask of row r (bit k: nbr[r,k] >= 0) for K <= 32, a 32-bit hash of the whole
 // pattern beyond (equal patterns still get equal keys); val[r] = r.
 __global__ void __launch_bounds__(128) row_keys_kernel(const int32_t* __restrict__ nbr, int64_t n, int K,
-                                                      uint32_t* __restrict__ keys, int32_t* __restrict__ vals) {
+                                                      uint32_t* __restrict__ keys, int32_t* __restrict__ vals,
+                                                      uint32_t* ticket) {
   extern __shared__ int32_t stage[];                     // 128 rows x K entries when K <= 64
+  if (ticket && blockIdx.x == 0 && threadIdx.x == 0) *ticket = 0;
   const int64_t row0 = (int64_t)blockIdx.x * 128;
   const int rows = (int)min((int64_t)128, n - row0);
   const int64_t row = row0 + threadIdx.x;
@@ -133,8 +135,9 @@ void sort_passes(const OrderScratch& s, int64_t n_rows, int K, int32_t* order, u
 }
 
 // ---- plan of the INVERSE map straight from the forward map (K <= 32), without writing the inverse ----
-__global__ void __launch_bounds__(256) iota_clear_kernel(uint32_t* keys, int32_t* vals, int64_t n) {
+__global__ void __launch_bounds__(256) iota_clear_kernel(uint32_t* keys, int32_t* vals, int64_t n, uint32_t* ticket) {
   const int64_t i = (int64_t)blockIdx.x * 256 + threadIdx.x;
+  if (ticket && i == 0) *ticket = 0;
   if (i < n) {
     keys[i] = 0u;
     vals[i] = (int32_t)i;
@@ -227,6 +230,168 @@ inverse_plan_scatter_kernel(const int32_t* __restrict__ nbr, int64_t n_flat, int
   }
 }
 
+// ---- balanced plans (K <= 32): the tiles in descending order of their number of offsets ----
+// The products hand tiles out in order to SMs that are free, so the big ones come first and the small ones fill up: with
+// the tiles in the order of their masks, the SM that got the last big one ended 1.1 to 1.6 times later than the mean.
+
+// A warp per tile: tmask[tile] = OR of its 128 sorted keys.  The block that finishes last ranks the tiles by a stable
+// counting sort, most offsets first (31 and 32 count alike); a tile that is not full keeps the last place.
+__global__ void __launch_bounds__(1024) tile_slots_kernel(const uint32_t* __restrict__ sorted_keys, int64_t n, int64_t n_tiles,
+                                                         uint32_t* tmask, int32_t* __restrict__ slot, uint32_t* ticket) {
+  __shared__ uint32_t next[32][33];                       // [warp][bin]
+  __shared__ uint32_t part[32];
+  __shared__ bool last;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int64_t tile = (int64_t)blockIdx.x * 32 + warp;
+  if (tile < n_tiles) {
+    uint32_t m = 0;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const int64_t at = tile * 128 + i * 32 + lane;
+      m |= at < n ? __ldg(sorted_keys + at) : 0u;
+    }
+    m = __reduce_or_sync(0xFFFFFFFFu, m);
+    if (lane == 0) tmask[tile] = m;
+  }
+  __threadfence();
+  __syncthreads();
+  if (threadIdx.x == 0) last = atomicAdd(ticket, 1u) == gridDim.x - 1;
+  next[warp][lane] = 0;
+  __syncthreads();
+  if (!last) return;
+  __threadfence();
+  const int64_t n_full = n / 128, per = ((n_full + 31) / 32 + 31) / 32 * 32;          // tiles of a warp
+  const int64_t begin = warp * per, end = min(n_full, begin + per);
+  const uint32_t lower = (1u << lane) - 1u;
+  constexpr int kBatch = 8;
+  auto each = [&](auto&& f) {                              // f(tile or -1, lanes of the same bin, bin)
+    for (int64_t t0 = begin; t0 < end; t0 += 32 * kBatch) {
+      uint32_t m[kBatch];
+#pragma unroll
+      for (int i = 0; i < kBatch; ++i) m[i] = t0 + i * 32 + lane < end ? __ldcg(tmask + t0 + i * 32 + lane) : 0u;
+#pragma unroll
+      for (int i = 0; i < kBatch; ++i) {
+        const int64_t t = t0 + i * 32 + lane;
+        const int bin = t < end ? 31 - min(__popc(m[i]), 31) : 32;
+        f(t < end ? t : -1, __match_any_sync(0xFFFFFFFFu, bin), bin);
+      }
+    }
+  };
+  each([&](int64_t t, uint32_t peers, int bin) {
+    if (t >= 0 && (peers & lower) == 0) next[warp][bin] += __popc(peers);
+    __syncwarp();
+  });
+  __syncthreads();
+  // first place of (bin, warp): thread = bin * 32 + warp of the count
+  const uint32_t count = next[lane][warp];
+  uint32_t upto = count;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const uint32_t u = __shfl_up_sync(0xFFFFFFFFu, upto, o);
+    if (lane >= o) upto += u;
+  }
+  if (lane == 31) part[warp] = upto;
+  __syncthreads();
+  const uint32_t before = __reduce_add_sync(0xFFFFFFFFu, lane < warp ? part[lane] : 0u);
+  next[lane][warp] = before + upto - count;
+  __syncthreads();
+  each([&](int64_t t, uint32_t peers, int bin) {
+    if (t >= 0) slot[t] = (int32_t)(next[warp][bin] + __popc(peers & lower));
+    __syncwarp();
+    if (t >= 0 && (peers & lower) == 0) next[warp][bin] += __popc(peers);
+    __syncwarp();
+  });
+  if (threadIdx.x == 0 && n_full < n_tiles) slot[n_full] = (int32_t)n_full;
+}
+
+// plan_tiles_kernel for K <= 32 with the masks and places of the tiles known: tile t of the sorted rows goes to place slot[t],
+// and only lines with a neighbour are written (nothing reads the others: a tenth of them is left at 3 offsets of 27).
+// Eight warps of 16 rows, all their loads in flight together; a row's K entries take 8, 16 or 32 lanes.
+__global__ void __launch_bounds__(256) plan_slots_kernel(const int32_t* __restrict__ nbr, const int32_t* __restrict__ sorted, int64_t n,
+                                                        int K, const uint32_t* __restrict__ sorted_mask,
+                                                        const int32_t* __restrict__ slots, int32_t* __restrict__ order,
+                                                        int32_t* __restrict__ tmap, uint32_t* __restrict__ tmask) {
+  __shared__ int32_t stage[128 * 33];
+  const int64_t tile = blockIdx.x, slot = __ldg(slots + tile);
+  const uint32_t mask = __ldg(sorted_mask + tile);
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int shift = K <= 8 ? 3 : K <= 16 ? 4 : 5, per_load = 32 >> shift;
+  const int k = lane & ((1 << shift) - 1), pitch = K | 1;
+  const int64_t pos = tile * 128 + warp * 16 + (lane & 15);
+  const int src = pos < n ? __ldg(sorted + pos) : -1;
+  if (lane < 16 && src >= 0) order[slot * 128 + warp * 16 + lane] = src;
+  if (threadIdx.x == 0) tmask[slot] = mask;
+  int32_t v[16];
+#pragma unroll
+  for (int i = 0; i < 16; ++i) {
+    const int row = i * per_load + (lane >> shift);
+    const int from = __shfl_sync(0xFFFFFFFFu, src, row & 15);
+    v[i] = i * per_load < 16 && from >= 0 && k < K ? __ldg(nbr + (int64_t)from * K + k) : -1;
+  }
+#pragma unroll
+  for (int i = 0; i < 16; ++i) {
+    const int row = i * per_load + (lane >> shift);
+    if (i * per_load < 16 && k < K) stage[(warp * 16 + row) * pitch + k] = v[i];
+  }
+  __syncthreads();
+  int turn = 0;
+  for (uint32_t m = mask; m; m &= m - 1, ++turn) {
+    if ((turn & 7) != warp) continue;
+    const int j = __ffs(m) - 1;
+    int32_t* line = tmap + (slot * K + j) * 128 + lane;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) line[i * 32] = stage[(i * 32 + lane) * pitch + j];
+  }
+}
+
+// The same for the inverse map, whose entries inverse_plan_scatter_kernel then fills in: the places of its rows, the row order,
+// the masks, and -1 in the lines that have a neighbour.
+__global__ void __launch_bounds__(128) inverse_slots_kernel(const int32_t* __restrict__ sorted, int64_t n, int K,
+                                                           const uint32_t* __restrict__ sorted_mask,
+                                                           const int32_t* __restrict__ slots, int32_t* __restrict__ rank,
+                                                           int32_t* __restrict__ order, int32_t* __restrict__ tmap,
+                                                           uint32_t* __restrict__ tmask) {
+  const int64_t tile = blockIdx.x, slot = __ldg(slots + tile), pos = tile * 128 + threadIdx.x;
+  const uint32_t mask = __ldg(sorted_mask + tile);
+  if (pos < n) {
+    const int row = __ldg(sorted + pos);
+    rank[row] = (int32_t)(slot * 128 + threadIdx.x);
+    order[slot * 128 + threadIdx.x] = row;
+  }
+  if (threadIdx.x == 0) tmask[slot] = mask;
+  for (uint32_t m = mask; m; m &= m - 1) tmap[(slot * K + __ffs(m) - 1) * 128 + threadIdx.x] = -1;
+}
+
+struct SlotScratch {
+  OrderScratch sort;
+  int32_t *rank, *slot;
+  uint32_t *mask, *ticket;
+};
+int64_t carve_slots(SlotScratch* s, void* ws, int64_t n, int K) {
+  int64_t off = carve(&s->sort, ws, n, K);
+  auto take = [&](int64_t count) {
+    char* p = ws ? static_cast<char*>(ws) + off : nullptr;
+    off += align_up((count > 0 ? count : 1) * 4, 256);
+    return p;
+  };
+  s->rank = reinterpret_cast<int32_t*>(take(n));
+  s->slot = reinterpret_cast<int32_t*>(take((n + 127) / 128));
+  s->mask = reinterpret_cast<uint32_t*>(take((n + 127) / 128));
+  s->ticket = reinterpret_cast<uint32_t*>(take(1));
+  return off;
+}
+// The sort of sort_passes, but with its result left in s.vals_b: `order` is the other buffer and is written afterwards.
+int32_t* first_vals_aside(const OrderScratch& s, int K, int32_t* order) { return passes_for(K) % 2 == 0 ? s.vals_b : order; }
+void sort_aside(const SlotScratch& s, int64_t n, int K, int32_t* order, cudaStream_t st) {
+  int32_t* vals_in = first_vals_aside(s.sort, K, order);
+  uint32_t* sorted_keys = nullptr;
+  radix_sort_pairs<uint32_t>(s.sort.keys_a, vals_in, s.sort.keys_b, vals_in == order ? s.sort.vals_b : order, n, K, s.sort.hist,
+                             s.sort.totals, &sorted_keys, nullptr, st);
+  const int64_t n_tiles = (n + 127) / 128;
+  tile_slots_kernel<<<(unsigned)((n_tiles + 31) / 32), 1024, 0, st>>>(sorted_keys, n, n_tiles, s.mask, s.slot, s.ticket);
+  note_launches(1);
+}
+
 }  // namespace
 
 }  // namespace st
@@ -256,7 +421,7 @@ int st_map_row_order(const int32_t* nbr, int64_t n_rows, int K, int32_t* order, 
   const size_t stage_bytes = K <= 64 ? (size_t)128 * K * 4 : 0;
   {
     row_keys_kernel<<<(unsigned)((n_rows + 127) / 128), 128, stage_bytes, st>>>(nbr, n_rows, K, s.keys_a,
-                                                                                first_vals(s, K, order));
+                                                                                first_vals(s, K, order), nullptr);
     note_launches(1);
   }
   sort_passes(s, n_rows, K, order, nullptr, st);
@@ -287,7 +452,7 @@ int st_map_plan_inverse(const int32_t* nbr, int64_t n_out, int K, int64_t n_in, 
   cudaStream_t st = (cudaStream_t)stream;
   const int64_t n_flat = n_out * K, n_tiles = (n_in + 127) / 128, n_tmap = n_tiles * K * 128;
   const unsigned rows_grid = (unsigned)((n_in + 255) / 256);
-  iota_clear_kernel<<<rows_grid, 256, 0, st>>>(s.keys_a, first_vals(s, K, order), n_in);
+  iota_clear_kernel<<<rows_grid, 256, 0, st>>>(s.keys_a, first_vals(s, K, order), n_in, nullptr);
   const unsigned flat_grid = (unsigned)((n_flat + kFlatPerBlock - 1) / kFlatPerBlock);
   const bool narrow = n_flat + kFlatPerBlock < 0x7FFFFFFFll;           // every flat index a thread forms fits 32 bits
   if (n_flat > 0) {
@@ -328,6 +493,64 @@ int st_map_plan(const int32_t* nbr, int64_t n_rows, int K, int sort_rows, int32_
     note_launches(1);
   }
   return check_launch("st_map_plan");
+}
+
+int64_t st_map_plan_balanced_workspace_bytes(int64_t n_rows, int K) {
+  SlotScratch s;
+  return carve_slots(&s, nullptr, n_rows, K);
+}
+
+int st_map_plan_balanced(const int32_t* nbr, int64_t n_rows, int K, int32_t* order, int32_t* tmap, uint32_t* tmask,
+                         void* workspace, int64_t workspace_bytes, void* stream) {
+  if (n_rows < 0 || K < 1 || K > 32 || n_rows > 0x7FFFFFFFll || (n_rows > 0 && (!nbr || !order || !tmap || !tmask || !workspace))) {
+    set_error("st_map_plan_balanced: bad arguments (K must be <= 32)");
+    return ST_ERR_ARG;
+  }
+  if (n_rows == 0) return ST_OK;
+  SlotScratch s;
+  if (workspace_bytes < carve_slots(&s, workspace, n_rows, K)) {
+    set_error("st_map_plan_balanced: workspace of %lld bytes is too small", (long long)workspace_bytes);
+    return ST_ERR_WORKSPACE;
+  }
+  cudaStream_t st = (cudaStream_t)stream;
+  const unsigned n_tiles = (unsigned)((n_rows + 127) / 128);
+  row_keys_kernel<<<n_tiles, 128, (size_t)128 * K * 4, st>>>(nbr, n_rows, K, s.sort.keys_a, first_vals_aside(s.sort, K, order), s.ticket);
+  sort_aside(s, n_rows, K, order, st);
+  plan_slots_kernel<<<n_tiles, 256, 0, st>>>(nbr, s.sort.vals_b, n_rows, K, s.mask, s.slot, order, tmap, tmask);
+  note_launches(2);
+  return check_launch("st_map_plan_balanced");
+}
+
+int st_map_plan_inverse_balanced(const int32_t* nbr, int64_t n_out, int K, int64_t n_in, int32_t* order, int32_t* tmap,
+                                 uint32_t* tmask, void* workspace, int64_t workspace_bytes, void* stream) {
+  if (n_out < 0 || n_in < 0 || K < 1 || K > 32 || n_in > 0x7FFFFFFFll || (n_out > 0 && !nbr) ||
+      (n_in > 0 && (!order || !tmap || !tmask || !workspace))) {
+    set_error("st_map_plan_inverse_balanced: bad arguments (K must be <= 32)");
+    return ST_ERR_ARG;
+  }
+  if (n_in == 0) return ST_OK;
+  SlotScratch s;
+  if (workspace_bytes < carve_slots(&s, workspace, n_in, K)) {
+    set_error("st_map_plan_inverse_balanced: workspace of %lld bytes is too small", (long long)workspace_bytes);
+    return ST_ERR_WORKSPACE;
+  }
+  cudaStream_t st = (cudaStream_t)stream;
+  const int64_t n_flat = n_out * K;
+  const bool narrow = n_flat + kFlatPerBlock < 0x7FFFFFFFll;
+  const unsigned flat_grid = (unsigned)((n_flat + kFlatPerBlock - 1) / kFlatPerBlock);
+  iota_clear_kernel<<<(unsigned)((n_in + 255) / 256), 256, 0, st>>>(s.sort.keys_a, first_vals_aside(s.sort, K, order), n_in, s.ticket);
+  if (n_flat > 0) {
+    if (narrow) inverse_keys_kernel<uint32_t><<<flat_grid, 256, 0, st>>>(nbr, n_flat, K, n_in, s.sort.keys_a);
+    else inverse_keys_kernel<int64_t><<<flat_grid, 256, 0, st>>>(nbr, n_flat, K, n_in, s.sort.keys_a);
+  }
+  sort_aside(s, n_in, K, order, st);
+  inverse_slots_kernel<<<(unsigned)((n_in + 127) / 128), 128, 0, st>>>(s.sort.vals_b, n_in, K, s.mask, s.slot, s.rank, order, tmap, tmask);
+  if (n_flat > 0) {
+    if (narrow) inverse_plan_scatter_kernel<uint32_t><<<flat_grid, 256, 0, st>>>(nbr, n_flat, K, n_in, s.rank, tmap);
+    else inverse_plan_scatter_kernel<int64_t><<<flat_grid, 256, 0, st>>>(nbr, n_flat, K, n_in, s.rank, tmap);
+  }
+  note_launches(4);
+  return check_launch("st_map_plan_inverse_balanced");
 }
 
 }  // extern "C"

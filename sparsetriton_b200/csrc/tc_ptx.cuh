@@ -166,6 +166,26 @@ __device__ __forceinline__ void mbar_arrive_expect_tx(uint32_t bar, uint32_t byt
   asm volatile("{\n\t.reg .b64 t;\n\tmbarrier.arrive.expect_tx.shared::cta.b64 t, [%0], %1;\n\t}" ::"r"(bar), "r"(bytes)
                : "memory");
 }
+// Ask for a CTA of this grid that has not started; the answer (16 bytes) arrives at `answer`, counted on `bar`.  Not to be
+// asked again once an answer said there is none.
+__device__ __forceinline__ void take_cta(uint32_t answer, uint32_t bar) {
+  asm volatile("clusterlaunchcontrol.try_cancel.async.shared::cta.mbarrier::complete_tx::bytes.b128 [%0], [%1];" ::"r"(answer),
+               "r"(bar) : "memory");
+}
+// The blockIdx.x that the answer gives this CTA, or -1.
+__device__ __forceinline__ int taken_cta(uint32_t answer) {
+  int cta;
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t.reg .b128 a;\n\t"
+      "ld.shared.b128 a, [%1];\n\t"
+      "clusterlaunchcontrol.query_cancel.is_canceled.pred.b128 p, a;\n\t"
+      "mov.s32 %0, -1;\n\t"
+      "@p clusterlaunchcontrol.query_cancel.get_first_ctaid::x.b32.b128 %0, a;\n\t}"
+      : "=r"(cta)
+      : "r"(answer)
+      : "memory");
+  return cta;
+}
 // Four rows of a 2-D tensor (row coordinates r0..r3, first column `col`) -> four consecutive 128-byte
 // lines at `dst`, written with the descriptor's swizzle; rows outside the tensor (e.g. -1) arrive as
 // zeros.  Completion is counted in bytes on `bar`.

@@ -47,8 +47,15 @@ const Plan& MapState::plan(const Tensor& nbr, bool row_order) {
   const cudaStream_t s = stream_of(nbr);
   Plan made;
   make_plan(&made, nbr, n, K, sorted, false);
-  Tensor ws = sorted ? bytes_on(nbr, st_map_plan_workspace_bytes(n, K)) : Tensor();
   Stage stage("map_plan", s);
+  if (sorted && K <= 32) {
+    Tensor ws = bytes_on(nbr, st_map_plan_balanced_workspace_bytes(n, K));
+    check(st_map_plan_balanced(nbr.data_ptr<int32_t>(), n, K, order_of(made), tmap_of(made), tmask_of(made), ws.data_ptr(),
+                               ws.numel(), s), "st_map_plan_balanced");
+    p = made;
+    return p;
+  }
+  Tensor ws = sorted ? bytes_on(nbr, st_map_plan_workspace_bytes(n, K)) : Tensor();
   check(st_map_plan(nbr.data_ptr<int32_t>(), n, K, sorted, order_of(made), tmap_of(made), tmask_of(made),
                     sorted ? ws.data_ptr() : nullptr, sorted ? ws.numel() : 0, s), "st_map_plan");
   p = made;
@@ -64,10 +71,10 @@ const Plan* MapState::inverse_plan(const Tensor& nbr, int64_t n_in, bool row_ord
   const cudaStream_t s = stream_of(nbr);
   Plan made;
   make_plan(&made, nbr, n_in, K, true, true);
-  Tensor ws = bytes_on(nbr, st_map_plan_inverse_workspace_bytes(n_in, K));
+  Tensor ws = bytes_on(nbr, st_map_plan_balanced_workspace_bytes(n_in, K));
   Stage stage("map_plan_inverse", s);
-  check(st_map_plan_inverse(nbr.data_ptr<int32_t>(), nbr.size(0), K, n_in, order_of(made), tmap_of(made), tmask_of(made),
-                            ws.data_ptr(), ws.numel(), s), "st_map_plan_inverse");
+  check(st_map_plan_inverse_balanced(nbr.data_ptr<int32_t>(), nbr.size(0), K, n_in, order_of(made), tmap_of(made), tmask_of(made),
+                            ws.data_ptr(), ws.numel(), s), "st_map_plan_inverse_balanced");
   inverse_plan_ = made;
   return &inverse_plan_;
 }

@@ -159,3 +159,42 @@ def test_pooling_forward_and_gradient(cuda_device, mode, C, grid, n):
         assert torch.allclose(torch.autograd.grad(out.F, x, dy)[0], torch.autograd.grad(want, x, dy)[0], atol=1e-6)
     finally:
         set_coords_dtype(before)
+
+
+@pytest.mark.parametrize("n_rows,n_src,K", [(1, 1, 1), (127, 90, 8), (128, 300, 9), (129, 129, 16), (5000, 4000, 27),
+                                            (40001, 30000, 32), (70000, 70001, 27), (1100000, 5000, 8)])
+def test_balanced_plans(cuda_device, n_rows, n_src, K):
+    """The plans that the products walk are those of st_map_plan(sorted) with whole tiles moved: most offsets first."""
+    L, dev, p = _lib.lib(), cuda_device, _lib.ptr
+    g = torch.Generator().manual_seed(n_rows + K)
+    nbr = torch.randint(0, n_src, (n_rows, K), generator=g, dtype=torch.int32)
+    nbr[torch.rand(n_rows, K, generator=g) > torch.rand(n_rows, 1, generator=g)] = -1
+    nbr = nbr.to(dev)
+    # a map that an inverse exists of: no source twice under one offset
+    fwd = torch.full((n_rows, K), -1, dtype=torch.int32, device=dev)
+    for k in range(K):
+        m = min(n_rows, n_src) // (1 + k % 5)
+        fwd[torch.randperm(n_rows, generator=g)[:m].to(dev), k] = torch.randperm(n_src, generator=g)[:m].to(dev, torch.int32)
+    inv = torch.empty((n_src, K), dtype=torch.int32, device=dev)
+    with torch.cuda.device(dev):
+        s = _lib.stream_ptr()
+        _lib.check(L.st_map_invert(p(fwd), n_rows, K, n_src, p(inv), s), "invert")
+        for of, n, call in ((nbr, n_rows, lambda b, w: L.st_map_plan_balanced(p(nbr), n_rows, K, *b, p(w), w.numel(), s)),
+                            (inv, n_src, lambda b, w: L.st_map_plan_inverse_balanced(p(fwd), n_rows, K, n_src, *b, p(w), w.numel(), s))):
+            tiles = (n + 127) // 128
+            plain, got = [[torch.full((m,), -7, dtype=torch.int32, device=dev) for m in (n, tiles * K * 128, tiles)] for _ in "ab"]
+            ws = _lib.workspace(L.st_map_plan_workspace_bytes(n, K), dev)
+            _lib.check(L.st_map_plan(p(of), n, K, 1, *[p(t) for t in plain], p(ws), ws.numel(), s), "plan")
+            ws = _lib.workspace(L.st_map_plan_balanced_workspace_bytes(n, K), dev)
+            _lib.check(call([p(t) for t in got], ws), "balanced")
+            bits = (plain[2][:, None] >> torch.arange(K, device=dev)) & 1
+            full = n // 128
+            place = torch.arange(tiles)
+            place[:full] = torch.sort(-bits[:full].sum(1).clamp(max=31).cpu(), stable=True).indices
+            place = place.to(dev)
+            assert torch.equal(got[2], plain[2][place])
+            assert torch.equal(got[0][:full * 128].view(-1, 128), plain[0][:full * 128].view(-1, 128)[place[:full]])
+            assert torch.equal(got[0][full * 128:], plain[0][full * 128:])
+            lines, want = got[1].view(tiles, K, 128), plain[1].view(tiles, K, 128)[place]
+            occupied = (bits[place] > 0)[:, :, None]
+            assert torch.equal(lines, torch.where(occupied, want, torch.full_like(want, -7)))
