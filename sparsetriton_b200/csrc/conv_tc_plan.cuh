@@ -9,7 +9,9 @@
 //
 // Warps 0-3 drain accumulators, warp 4 issues the MMAs, warp 5 fetches W slices by TMA, warps 6-21 fetch rows with
 // 16-byte cp.async: four groups of four warps take the stages in turn, a warp has 32 rows of a stage.  Warp 22 hands out
-// super tiles with their tile masks, which the others walk themselves.
+// super tiles with their tile masks, which the MMA and W warps walk themselves, and lists their stages for the row warps:
+// with the walk in all sixteen of them, it was two thirds of their instructions, and without any copy, store or W slice the
+// kernel still took 135 of 170 us (815249 rows, 64 -> 128).
 //
 // Who does which super tile: super tiles cost 1 to K offsets, and dealt out in a fixed pattern the busiest SM had 1.3 to 2
 // times the mean.  The grid is one CTA per super tile, and a CTA that runs takes over others before they start
@@ -35,7 +37,7 @@ constexpr int kWarpW = kMmaWarp + 1;                          // the warp that f
 constexpr int kFirstRowWarp = kWarpW + 1;
 constexpr int kWarpJobs = kFirstRowWarp + kRowGroups * kRowGroupWarps;
 constexpr int kGather3Threads = (kWarpJobs + 1) * 32;
-constexpr int kJobReaders = kWarpJobs;                        // all warps before it
+constexpr int kJobReaders = kFirstRowWarp;
 // Super tiles on offer at a time.  Every one taken early is one that cannot go to an SM that turns out to be free.
 constexpr int kJobs = 2;
 
@@ -45,16 +47,63 @@ struct Job {
   uint32_t mask[kMaxSub];                                      // offsets 0 .. 31
 };
 
+// Up to 32 stages of one super tile: the index line of each and its column block of the reduction.
+struct Batch {
+  uint2 entry[32];
+  int n;                                                       // -1: no more
+};
+constexpr int kBatches = 4;
+
 struct __align__(8) Control3 {
   unsigned long long a_full[kMaxAStages], a_empty[kMaxAStages];
   unsigned long long w_full[kMaxWSlots], w_empty[kMaxWSlots];
   unsigned long long acc_full[2], acc_empty[2];
   unsigned long long job_full[kJobs], job_empty[kJobs], taken;
+  unsigned long long batch_full[kBatches], batch_empty[kBatches];
   __align__(16) uint4 taken_cta;
+  Batch batch[kBatches];
   Job job[kJobs];
   uint32_t tmem_base;
   int abort_flag;
 };
+
+static_assert(sizeof(Control3) <= 2048, "see the shared memory budget in fill_params2");
+struct BatchWriter {
+  Control3* ctl;
+  volatile int* abort_flag;
+  int lane;
+  int slot = 0;
+  uint32_t phase = 0;
+  __device__ __forceinline__ bool put(uint2 entry, int n) {
+    if (!mbar_wait_all(smem_u32(&ctl->batch_empty[slot]), phase ^ 1u, abort_flag, 45)) return false;
+    ctl->batch[slot].entry[lane] = entry;
+    if (lane == 0) ctl->batch[slot].n = n;
+    __syncwarp();
+    if (lane == 0) mbar_arrive(smem_u32(&ctl->batch_full[slot]));
+    if (++slot == kBatches) {
+      slot = 0;
+      phase ^= 1u;
+    }
+    return true;
+  }
+};
+// Every lane has a count; the inclusive sums of the counts, and the lane that output `o` belongs to.
+__device__ __forceinline__ uint32_t lane_sums(uint32_t count, int lane) {
+#pragma unroll
+  for (int d = 1; d < 32; d <<= 1) {
+    const uint32_t before = __shfl_up_sync(0xFFFFFFFFu, count, d);
+    if (lane >= d) count += before;
+  }
+  return count;
+}
+__device__ __forceinline__ int owner_of(uint32_t upto, uint32_t o) {
+  int l = 0;
+#pragma unroll
+  for (int step = 16; step; step >>= 1) {
+    if (__shfl_sync(0xFFFFFFFFu, upto, l + step - 1) <= o) l += step;
+  }
+  return l;
+}
 
 // A warp's view of the super tiles this CTA has, in order.
 struct JobReader {
@@ -64,10 +113,7 @@ struct JobReader {
   int slot = 0;
   uint32_t phase = 0;
   Job job;
-  // before_wait(): what others may need from this warp before the next job can come.
-  template <typename F>
-  __device__ __forceinline__ bool next(F&& before_wait) {
-    if (!__all_sync(0xFFFFFFFFu, mbar_try_now(smem_u32(&ctl->job_full[slot]), phase))) before_wait();
+  __device__ __forceinline__ bool next() {
     if (!mbar_wait_all(smem_u32(&ctl->job_full[slot]), phase, abort_flag, 43)) return false;
     job = ctl->job[slot];
     __syncwarp();
@@ -83,10 +129,10 @@ struct JobReader {
 // The work of this CTA in order: item(tile0, k, kb, users, fresh) for every occupied (offset, 128-byte block) of a
 // super tile (users: the sub tiles that have the offset; fresh: those whose accumulator starts here), between
 // begin(tile0) and end(tile0).  Stops when one of them returns false.
-template <typename Idle, typename Begin, typename Item, typename End>
+template <typename Begin, typename Item, typename End>
 __device__ __forceinline__ void walk_super_tiles(const Params2& p, const PlannedRows& map, int64_t n_tiles, JobReader jobs,
-                                                 Idle&& before_wait, Begin&& begin, Item&& item, End&& end) {
-  while (jobs.next(before_wait)) {
+                                                 Begin&& begin, Item&& item, End&& end) {
+  while (jobs.next()) {
     const int64_t tile0 = (int64_t)jobs.job.super * p.sub;
     // every lane has the same words; the reduction tells the compiler so (uniform registers and branches)
     uint32_t m[kMaxSub];
@@ -219,6 +265,10 @@ __global__ void __launch_bounds__(kGather3Threads, 1) planned_gather_kernel(cons
       mbar_init(smem_u32(&ctl->acc_full[b]), 1);
       mbar_init(smem_u32(&ctl->acc_empty[b]), kEpilogueWarps * 32);
     }
+    for (int s = 0; s < kBatches; ++s) {
+      mbar_init(smem_u32(&ctl->batch_full[s]), 1);
+      mbar_init(smem_u32(&ctl->batch_empty[s]), kRowGroups * kRowGroupWarps);
+    }
     for (int s = 0; s < kJobs; ++s) {
       mbar_init(smem_u32(&ctl->job_full[s]), 1);
       mbar_init(smem_u32(&ctl->job_empty[s]), kJobReaders);
@@ -245,6 +295,7 @@ __global__ void __launch_bounds__(kGather3Threads, 1) planned_gather_kernel(cons
     // =============================================================== super tiles
     int super = blockIdx.x, slot = 0;
     uint32_t phase = 0, taken_phase = 0;
+    BatchWriter batches{ctl, abort_flag, lane};
     while (true) {
       if (!mbar_wait_all(smem_u32(&ctl->job_empty[slot]), phase ^ 1u, abort_flag, 41)) break;
       if (super < 0) {                                         // not the first: take over a CTA that has not started
@@ -273,16 +324,40 @@ __global__ void __launch_bounds__(kGather3Threads, 1) planned_gather_kernel(cons
       }
       __syncwarp();
       if (lane == 0) mbar_arrive(smem_u32(&ctl->job_full[slot]));
-      if (super < 0) break;
-      // its index lines: have them in L2 by the time the row warps ask
-      for (int s = 0; s < p.sub; ++s) {
-        const uint32_t m = __shfl_sync(0xFFFFFFFFu, mask, s);
-        if ((m >> lane) & 1u) {
-          const char* line = reinterpret_cast<const char*>(map.tmap + (((int64_t)super * p.sub + s) * map.K + lane) * kTileM);
+      // its stages: offset by offset, column block by column block, the sub tiles that have the offset in turn
+      bool ok = true;
+      for (int word = 0; word < map.MW && super >= 0 && ok; ++word) {
+        if (word) mask = lane < p.sub && tile < n_tiles ? __ldg(map.tmask + tile * map.MW + word) : 0u;
+        uint32_t users = 0;                                    // lane = offset
 #pragma unroll
-          for (int i = 0; i < 4; ++i) prefetch_l2(line + i * 128);
+        for (int s = 0; s < kMaxSub; ++s) users |= ((__shfl_sync(0xFFFFFFFFu, mask, s) >> lane) & 1u) << s;
+        const uint32_t upto = lane_sums((uint32_t)(__popc(users) * p.k_blocks), lane);
+        const uint32_t total = __shfl_sync(0xFFFFFFFFu, upto, 31);
+        for (uint32_t o0 = 0; o0 < total && ok; o0 += 32) {
+          const uint32_t o = min(o0 + lane, total - 1);        // lane = stage
+          const int j = owner_of(upto, o);
+          uint32_t u = __shfl_sync(0xFFFFFFFFu, users, j);
+          const uint32_t n_users = (uint32_t)__popc(u);
+          const uint32_t at = o - (__shfl_sync(0xFFFFFFFFu, upto, j) - n_users * (uint32_t)p.k_blocks);
+          const uint32_t kb = at / n_users, which = at - kb * n_users;
+#pragma unroll
+          for (uint32_t q = 0; q + 1 < kMaxSub; ++q)
+            if (q < which) u &= u - 1;
+          const uint32_t line = (uint32_t)(((int64_t)super * p.sub + __ffs(u) - 1) * map.K + word * 32 + j);
+          const int n = (int)min(32u, total - o0);
+          if (kb == 0 && lane < n) {                           // have it in L2 by the time the row warps ask
+            const char* at_line = reinterpret_cast<const char*>(map.tmap) + (size_t)line * (kTileM * 4);
+#pragma unroll
+            for (int i = 0; i < 4; ++i) prefetch_l2(at_line + i * 128);
+          }
+          ok = batches.put(make_uint2(line, kb), n);
         }
       }
+      if (super < 0) {
+        if (ok) batches.put(make_uint2(0u, 0u), -1);
+        break;
+      }
+      if (!ok) break;
       super = -1;
       if (++slot == kJobs) {
         slot = 0;
@@ -291,13 +366,13 @@ __global__ void __launch_bounds__(kGather3Threads, 1) planned_gather_kernel(cons
     }
   } else if (warp >= kFirstRowWarp) {
     // =============================================================== rows
-    static_assert(kRowGroups == kMaxSub, "an offset has at most one stage per group");
     const int group = (warp - kFirstRowWarp) / kRowGroupWarps;
     const int row0 = (warp - kFirstRowWarp) % kRowGroupWarps * 32;
     const char* in = static_cast<const char*>(p.in);
     int sent = -1;                                            // stage whose copies are under way, not yet announced
-    int stage = 0, turn = 0;                                  // ring position and group of the next stage
+    int first = group, next = group;                          // a_stages > kRowGroups: every group starts in the first lap
     uint32_t phase = 0;
+    const int32_t* lines = map.tmap + row0 + lane;
     bool ok = true;
     int pend_stage = -1, pend_kb = 0, pend_idx = -1;
     uint32_t pend_parity = 0;
@@ -314,7 +389,7 @@ __global__ void __launch_bounds__(kGather3Threads, 1) planned_gather_kernel(cons
       sent = pend_stage;
     };
     auto flush = [&]() {
-      // the job that this warp is about to wait for may wait for the stages that it has not announced
+      // the batch that this warp is about to wait for may wait for the stages that it has not announced
       if (pend_stage >= 0 && ok) run();
       pend_stage = -1;
       cp_async_wait_all();
@@ -323,30 +398,41 @@ __global__ void __launch_bounds__(kGather3Threads, 1) planned_gather_kernel(cons
       if (sent >= 0 && lane == 0) mbar_arrive(smem_u32(&ctl->a_full[sent]));
       sent = -1;
     };
-    walk_super_tiles(p, map, n_tiles, jobs, flush, nothing, [&](int64_t tile0, int k, int kb, uint32_t users, uint32_t) {
-      const int n = __popc(users), mine = (group - turn) & (kRowGroups - 1);
-      if (mine < n) {
-        // this stage's row numbers are loaded now and its copies issued when the group's next stage comes up, so that
+    int slot = 0;
+    uint32_t slot_phase = 0;
+    while (ok) {
+      const uint32_t full = smem_u32(&ctl->batch_full[slot]);
+      if (!__all_sync(0xFFFFFFFFu, mbar_try_now(full, slot_phase))) flush();
+      if (!ok || !mbar_wait_all(full, slot_phase, abort_flag, 44)) break;
+      const int n = ctl->batch[slot].n;
+      const uint2 entry = ctl->batch[slot].entry[lane];        // lane = stage
+      __syncwarp();
+      if (lane == 0) mbar_arrive(smem_u32(&ctl->batch_empty[slot]));
+      if (++slot == kBatches) {
+        slot = 0;
+        slot_phase ^= 1u;
+      }
+      if (n < 0) break;
+      // this group's are the stages first, first + 4, ...; `next` and `phase`: ring position of the group's next one
+      int e = first;
+      for (; e < n && ok; e += kRowGroups) {
+        // a stage's row numbers are loaded now and its copies issued when the group's next stage comes up, so that
         // the load overlaps the wait and copies of the one before
-        uint32_t u = users;
-        for (int i = 0; i < mine; ++i) u &= u - 1;
-        const int s = __ffs(u) - 1;
-        const int idx = __ldg(map.tmap + ((tile0 + s) * map.K + k) * (int64_t)kTileM + row0 + lane);
+        const uint32_t line = __shfl_sync(0xFFFFFFFFu, entry.x, e);
+        const int idx = __ldg(lines + (size_t)line * kTileM);
         if (pend_stage >= 0) run();
-        const bool wrap = stage + mine >= p.a_stages;
-        pend_stage = wrap ? stage + mine - p.a_stages : stage + mine;
-        pend_parity = wrap ? phase ^ 1u : phase;
-        pend_kb = kb;
+        pend_stage = next;
+        pend_parity = phase;
+        pend_kb = (int)__shfl_sync(0xFFFFFFFFu, entry.y, e);
         pend_idx = idx;
+        next += kRowGroups;
+        if (next >= p.a_stages) {
+          next -= p.a_stages;
+          phase ^= 1u;
+        }
       }
-      turn = (turn + n) & (kRowGroups - 1);
-      stage += n;
-      if (stage >= p.a_stages) {
-        stage -= p.a_stages;
-        phase ^= 1u;
-      }
-      return ok;
-    }, nothing);
+      first = e - n;
+    }
     flush();
   } else if (warp == kWarpW) {
     // =============================================================== W slices
@@ -355,7 +441,7 @@ __global__ void __launch_bounds__(kGather3Threads, 1) planned_gather_kernel(cons
     const uint32_t w_bytes = p.b_mn_major ? (uint32_t)(((w_col_bytes + 127) >> 7) * kr * 128) : (uint32_t)(p.w_rows * 128);
     int slot = 0;
     uint32_t phase = 0;
-    walk_super_tiles(p, map, n_tiles, jobs, [] {}, nothing, [&](int64_t, int k, int kb, uint32_t, uint32_t) {
+    walk_super_tiles(p, map, n_tiles, jobs, nothing, [&](int64_t, int k, int kb, uint32_t, uint32_t) {
       if (!mbar_wait_all(smem_u32(&ctl->w_empty[slot]), phase ^ 1u, abort_flag, 35)) return false;
       if (lane == 0) {
         const uint32_t bar = smem_u32(&ctl->w_full[slot]);
@@ -394,7 +480,7 @@ __global__ void __launch_bounds__(kGather3Threads, 1) planned_gather_kernel(cons
       const uint64_t a_desc_hi = smem_desc(0u, 16u, 1024u, 2u);
       const uint64_t b_desc_hi = smem_desc(0u, b_lbo, b_base32 ? 512u : 1024u, b_base32 ? 1u : 2u);
       const uint32_t idesc = p.idesc;
-      walk_super_tiles(p, map, n_tiles, jobs, [] {},
+      walk_super_tiles(p, map, n_tiles, jobs,
         [&](int64_t) {
           const bool ok = mbar_wait_all(smem_u32(&ctl->acc_empty[buf]), acc_phase[buf] ^ 1u, abort_flag, 32);
           tc_fence_after();
@@ -457,7 +543,7 @@ __global__ void __launch_bounds__(kGather3Threads, 1) planned_gather_kernel(cons
     const int out_es = p.out_kind == ST_F32 ? 4 : 2;
     const uint32_t stage_rows = out_ring + (uint32_t)warp * kOutWarpBytes;
     JobReader mine = jobs;
-    while (ok && mine.next([] {})) {
+    while (ok && mine.next()) {
       const int64_t st_i = mine.job.super;
       // where this lane's rows go: known before the accumulators are ready, so fetched before the wait
       int64_t dst_rows[kMaxSub];
