@@ -626,6 +626,8 @@ map_build_columns_kernel(const CT* __restrict__ coords, int64_t n_threads, CubeO
   if (x < 0 || x >= shape.x || y < 0 || y >= shape.y || table.capacity == 0 || !key_representable(c.x, x, y, 0)) return;
   const int last = col == kCols - 1 ? KS / 2 : KS - 1;         // the centre column: up to the row itself
   const bool inside = c.y >= 0 && c.y < shape.x && c.z >= 0 && c.z < shape.y && c.w >= 0 && c.w < shape.z;
+  // the filter's answers first, all of them, then the probes that are left
+  uint32_t want = 0;                                           // bit iz
   int have = -1;                                               // block whose bits are at hand
   uint32_t bits = 0;
 #pragma unroll
@@ -636,8 +638,12 @@ map_build_columns_kernel(const CT* __restrict__ coords, int64_t n_threads, CubeO
       have = z >> 5;
       bits = __ldg(filter.word(c.x, x, y, z));
     }
-    if (!((bits >> (z & 31)) & 1u)) continue;
-    const int32_t r = table_find(table, pack_key(c.x, x, y, z));
+    want |= ((bits >> (z & 31)) & 1u) << iz;
+  }
+#pragma unroll 1
+  for (; want; want &= want - 1) {
+    const int iz = __ffs(want) - 1;
+    const int32_t r = table_find(table, pack_key(c.x, x, y, c.w - cube.at(2, iz)));
     if (r < 0) continue;
     const int k = k0 + iz;
     nbr[row * K + k] = r;

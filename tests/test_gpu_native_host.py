@@ -1,5 +1,7 @@
 """The native host side and the kernels behind it at the sizes where they can go wrong: edges of tiles and rings, remainders,
 the smallest and largest of a range.  References are plain PyTorch in fp32, or the slower form of the same entry point."""
+import ctypes
+
 import pytest
 import torch
 
@@ -198,3 +200,37 @@ def test_balanced_plans(cuda_device, n_rows, n_src, K):
             lines, want = got[1].view(tiles, K, 128), plain[1].view(tiles, K, 128)[place]
             occupied = (bits[place] > 0)[:, :, None]
             assert torch.equal(lines, torch.where(occupied, want, torch.full_like(want, -7)))
+
+
+@pytest.mark.parametrize("ks,n", [(3, 1500000), (5, 200000), (7, 60000)])
+def test_filtered_map_is_the_probed_map(cuda_device, ks, n):
+    """st_map_build_symmetric_ws with the column filter's workspace and without it, over tables whose chains differ from one
+    build to the next (rows claim their slots in any order)."""
+    L, dev, p = _lib.lib(), cuda_device, _lib.ptr
+    g = torch.Generator(device=dev).manual_seed(ks)
+    flat = torch.randint(0, 16 * 400 * 400, (n // 4,), generator=g, device=dev)              # short columns: surfaces
+    z0 = torch.randint(0, 37, (n // 4,), generator=g, device=dev)
+    c = torch.stack([flat // 160000, flat // 400 % 400, flat % 400, z0], 1).repeat_interleave(4, 0)
+    c[:, 3] += torch.arange(4, device=dev).repeat(n // 4)
+    c = torch.unique(c, dim=0).int().contiguous()
+    n = c.shape[0]
+    r, K = ks // 2, ks ** 3
+    offs = [v for x in range(r, -r - 1, -1) for y in range(r, -r - 1, -1) for z in range(r, -r - 1, -1) for v in (x, y, z)]
+    off, shape = (ctypes.c_int32 * (3 * K))(*offs), (ctypes.c_int32 * 3)(400, 400, 41)
+    need = L.st_map_build_symmetric_workspace_bytes(n, K)
+    assert need > 0
+    ws = torch.empty(need, dtype=torch.uint8, device=dev)
+    cap = 1 << (2 * n - 1).bit_length()
+    keys, vals = torch.empty(cap, dtype=torch.int64, device=dev), torch.empty(cap, dtype=torch.int32, device=dev)
+    status = torch.zeros(1, dtype=torch.int32, device=dev)
+    a, b = (torch.empty((n, K), dtype=torch.int32, device=dev) for _ in "ab")
+    code = _lib.coord_code(c)
+    with torch.cuda.device(dev):
+        s = _lib.stream_ptr()
+        for _ in range(8):
+            _lib.check(L.st_hash_clear(p(keys), p(vals), cap, s), "clear")
+            _lib.check(L.st_hash_build(p(c), n, code, p(keys), p(vals), cap, p(status), s), "build")
+            for out, w in ((a, ws), (b, None)):
+                _lib.check(L.st_map_build_symmetric_ws(p(c), n, code, off, K, shape, p(keys), p(vals), cap, p(out), None,
+                                                       p(w) if w is not None else None, need if w is not None else 0, s), "map")
+            assert torch.equal(a, b)
