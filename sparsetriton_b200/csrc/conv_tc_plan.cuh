@@ -602,7 +602,9 @@ __global__ void __launch_bounds__(kGather3Threads, 1) planned_gather_kernel(cons
 // A CTA owns a group of G offsets (G accumulators fill TMEM), a block of output and one of input channels, and a share
 // of the row tiles.  Per tile that has an offset of the group it brings in the tile operand (128 rows of dY, picked through
 // `order`) once and the gathered operand (128 rows of X through the tile's index line) per offset; both come with 16-byte
-// cp.async from 16 warps, as in planned_gather_kernel, through two rings.  With p.swap the plan is the INVERSE map's: the
+// cp.async from 16 warps, as in planned_gather_kernel, through two rings, and announce themselves (an asynchronous arrival per
+// thread): a warp that announced an item when its next one was on its way held back the two or three tile slots (256 -> 256,
+// 95541 rows: 385 -> 340 us; two or three items held back: 440, 460).  With p.swap the plan is the INVERSE map's: the
 // tile operand is X and the gathered one dY.
 //
 // How the CTAs are shared out: an odd kernel's centre offset occurs in every tile of a submanifold layer and the others in
@@ -670,11 +672,11 @@ __global__ void __launch_bounds__(kWgrad3Threads, 1) planned_wgrad_kernel(const 
   for (int g = threadIdx.x; g < p.n_kgroups; g += kWgrad3Threads) ctl->weight[g] = 0;
   if (threadIdx.x == 0) {
     for (int s = 0; s < p.a_slots; ++s) {
-      mbar_init(smem_u32(&ctl->a_full[s]), kRowGroups * kRowGroupWarps);
+      mbar_init(smem_u32(&ctl->a_full[s]), kRowGroups * kRowGroupWarps * 32);
       mbar_init(smem_u32(&ctl->a_empty[s]), 1);
     }
     for (int s = 0; s < p.b_slots; ++s) {
-      mbar_init(smem_u32(&ctl->b_full[s]), kRowGroupWarps);
+      mbar_init(smem_u32(&ctl->b_full[s]), kRowGroupWarps * 32);
       mbar_init(smem_u32(&ctl->b_empty[s]), 1);
     }
     mbar_init(smem_u32(&ctl->acc_full), 2);
@@ -764,22 +766,11 @@ __global__ void __launch_bounds__(kWgrad3Threads, 1) planned_wgrad_kernel(const 
     int a_slot = 0, b_slot = 0, turn = 0;
     uint32_t a_phase = 0, b_phase = 0;
     bool ok = true;
-    uint32_t sent = 0;                                        // barrier of the item whose copies are under way, not yet announced
     bool pend = false, pend_b = false;
     int pend_slot = 0, pend_idx = -1;
     uint32_t pend_parity = 0;
-    auto announce = [&]() {
-      __syncwarp();
-      if (sent && lane == 0) mbar_arrive(sent);
-      sent = 0;
-    };
     auto wait_for = [&](bool is_b, int slot, uint32_t parity) {
-      const uint32_t empty = smem_u32(is_b ? &ctl->b_empty[slot] : &ctl->a_empty[slot]);
-      if (__all_sync(0xFFFFFFFFu, mbar_try_now(empty, parity ^ 1u))) return true;
-      // the slot's release may depend on what this warp has not announced yet
-      cp_async_wait_all();
-      announce();
-      return mbar_wait_all(empty, parity ^ 1u, abort_flag, is_b ? 36 : 35);
+      return mbar_wait_all(smem_u32(is_b ? &ctl->b_empty[slot] : &ctl->a_empty[slot]), parity ^ 1u, abort_flag, is_b ? 36 : 35);
     };
     auto run = [&]() {
       ok = wait_for(pend_b, pend_slot, pend_parity);
@@ -795,10 +786,7 @@ __global__ void __launch_bounds__(kWgrad3Threads, 1) planned_wgrad_kernel(const 
           fetch_block<8, kBase32>(dst + (uint32_t)b * kABlockBytes, t_row0, pend_idx, t_src + b * 128, t_pitch, p.n_rows,
                                   min(128, t_bytes - b * 128), lane);
       }
-      cp_async_commit();
-      cp_async_wait_group<1>();                               // the item before this one has landed: announce it
-      announce();
-      sent = smem_u32(pend_b ? &ctl->b_full[pend_slot] : &ctl->a_full[pend_slot]);
+      cp_async_arrive_noinc(smem_u32(pend_b ? &ctl->b_full[pend_slot] : &ctl->a_full[pend_slot]));      // when they have landed
     };
     auto queue = [&](bool is_b, int slot, uint32_t parity, int idx) {
       if (pend) run();
@@ -835,30 +823,36 @@ __global__ void __launch_bounds__(kWgrad3Threads, 1) planned_wgrad_kernel(const 
     });
     if (pend && ok) run();
     cp_async_wait_all();
-    announce();
   } else if (warp == kMmaWarp) {
     // =============================================================== MMA issuer (see planned_gather_kernel)
     int a_slot = 0, b_slot = 0;
     uint32_t a_phase = 0, b_phase = 0;
     uint32_t touched = 0;
     bool ok = true;
+    bool a_ready = false, b_ready = false;                     // what a look ahead at the next slots said
     constexpr int kRowsPerStep = 32 / ESIZE;                   // reduction rows per MMA (16 or 8)
     constexpr int kSteps = kTileM / kRowsPerStep;
     constexpr uint32_t kStep16 = kRowsPerStep * 128 / 16;
     const uint32_t idesc = p.idesc_base | ((uint32_t)(p.ci_blk >> 3) << 17);
     const uint64_t desc_hi = smem_desc(0u, kABlockBytes, kBase32 ? 512u : 1024u, kBase32 ? 1u : 2u);
     walk_tiles(p, map, tile_begin, tile_step, word, shift, group_bits, lane, [&](int64_t, uint32_t m) {
-      ok = mbar_wait_all(smem_u32(&ctl->a_full[a_slot]), a_phase, abort_flag, 37);
+      ok = __all_sync(0xFFFFFFFFu, a_ready) || mbar_wait_all(smem_u32(&ctl->a_full[a_slot]), a_phase, abort_flag, 37);
       if (!ok) return false;
       const uint32_t t_lo = (a_ring + (uint32_t)a_slot * (uint32_t)p.a_slot_bytes) >> 4;
       while (m) {
         const int j = __ffs(m) - 1;
         m &= m - 1;
-        ok = mbar_wait_all(smem_u32(&ctl->b_full[b_slot]), b_phase, abort_flag, 38);
+        ok = __all_sync(0xFFFFFFFFu, b_ready) || mbar_wait_all(smem_u32(&ctl->b_full[b_slot]), b_phase, abort_flag, 38);
         if (!ok) return false;
+        const int this_slot = b_slot;
+        if (++b_slot == p.b_slots) {
+          b_slot = 0;
+          b_phase ^= 1u;
+        }
+        b_ready = mbar_try_now(smem_u32(&ctl->b_full[b_slot]), b_phase);
         fence_proxy_async();                                   // rows were written by cp.async
         tc_fence_after();
-        const uint32_t g_lo = (b_ring + (uint32_t)b_slot * (uint32_t)p.b_slot_bytes) >> 4;
+        const uint32_t g_lo = (b_ring + (uint32_t)this_slot * (uint32_t)p.b_slot_bytes) >> 4;
         const uint32_t a_lo = p.swap ? g_lo : t_lo, b_lo = p.swap ? t_lo : g_lo;   // dY rows (M), X rows (N)
         const uint32_t d_addr = tmem_base + (uint32_t)(j * p.ci_blk);
         const uint32_t add = (touched >> j) & 1u;
@@ -872,19 +866,16 @@ __global__ void __launch_bounds__(kWgrad3Threads, 1) planned_wgrad_kernel(const 
             else
               mma_tf32(d_addr, da, db, idesc, ks == 0 ? add : 1u);
           }
-          mma_commit(smem_u32(&ctl->b_empty[b_slot]));
+          mma_commit(smem_u32(&ctl->b_empty[this_slot]));
         }
         touched |= 1u << j;
-        if (++b_slot == p.b_slots) {
-          b_slot = 0;
-          b_phase ^= 1u;
-        }
       }
       if (elect_one()) mma_commit(smem_u32(&ctl->a_empty[a_slot]));
       if (++a_slot == p.a_slots) {
         a_slot = 0;
         a_phase ^= 1u;
       }
+      a_ready = mbar_try_now(smem_u32(&ctl->a_full[a_slot]), a_phase);
       return true;
     });
     if (ok && elect_one()) {

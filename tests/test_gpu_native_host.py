@@ -150,7 +150,8 @@ def test_pooling_forward_and_gradient(cuda_device, mode, C, grid, n):
     set_coords_dtype(torch.int32)
     try:
         c = synthetic.random_cells(n, 2, grid, seed=n).to(cuda_device)
-        x = torch.randn(n, C, device=cuda_device, requires_grad=True)
+        x = (torch.randperm(n * C, device=cuda_device).float() * 2.0 ** -20 - 0.5).view(n, C)      # no ties under a maximum
+        x.requires_grad_(True)
         out = sparse_pooling(SparseTensor(x, c, (grid,) * 3, 2), 4, 2, 4, mode)
         key = ((c[:, 0].long() * 64 + c[:, 1] // 4) * 64 + c[:, 2] // 4) * 64 + c[:, 3] // 4
         cells, inv = torch.unique(key, return_inverse=True)
