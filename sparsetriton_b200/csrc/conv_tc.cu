@@ -1293,8 +1293,8 @@ static int launch_gather(tc::Params2 p, const Map& map, cudaStream_t stream) {
   return check_launch("tc gather");
 }
 
-// A stored map in tile-plan form.  A row warp announces a stage when its group's next one is under way, so the ring must be
-// longer than the number of groups.  planned_gather_kernel when the weights can be described to the copy engine and the
+// A stored map in tile-plan form.  A wait names a lap of the ring by its parity, and a group of row warps knows which lap the
+// MMAs are in from the stage it filled before: the ring must be longer than the number of groups.  planned_gather_kernel when the weights can be described to the copy engine and the
 // rows are whole 16-byte pieces, else gather2_kernel over the same plan.
 static int launch_planned(tc::Params2 p, const tc::PlannedRows& map, cudaStream_t stream) {
   CUtensorMap w_desc;
