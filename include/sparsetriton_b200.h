@@ -479,6 +479,16 @@ int st_conv_wgrad_hashfly(int dtype, const void* X, const void* dY, const void* 
                           int64_t n_out, int K, int cin, int cout, void* workspace, int64_t workspace_bytes,
                           void* stream);
 
+/* Per-voxel linear head: y (n, O) fp32 = x (n, C) W^T + bias with W (O, C) and bias (O,) in fp32, x of `dtype`; bias may be NULL.
+ * st_linear_dgrad: dx (of `dtype`) = dy W.  st_linear_wgrad: dw = dy^T x and, unless NULL, db = column sums of dy; sums in a
+ * fixed order.  C of 16, 32 or 64, O a multiple of 4 up to 64 (st_linear_supported); x, dx, y and dy 16-byte aligned. */
+int st_linear_supported(int dtype, int C, int O);
+int st_linear_fwd(int dtype, const void* x, const float* w, const float* bias, float* y, int64_t n, int C, int O, void* stream);
+int st_linear_dgrad(int dtype, const float* dy, const float* w, void* dx, int64_t n, int C, int O, void* stream);
+int64_t st_linear_workspace_bytes(int64_t n, int C, int O);
+int st_linear_wgrad(int dtype, const void* x, const float* dy, float* dw, float* db, int64_t n, int C, int O, void* workspace,
+                    int64_t workspace_bytes, void* stream);
+
 #ifdef __cplusplus
 }
 #endif

@@ -75,6 +75,11 @@ _SIGNATURES["st_map_plan_inverse"] = ([_PTR, _I64, _INT, _I64, _PTR, _PTR, _PTR,
 _SIGNATURES["st_map_plan_balanced_workspace_bytes"] = ([_I64, _INT], _I64)
 _SIGNATURES["st_map_plan_balanced"] = ([_PTR, _I64, _INT, _PTR, _PTR, _PTR, _PTR, _I64, _PTR], _INT)
 _SIGNATURES["st_map_plan_inverse_balanced"] = _SIGNATURES["st_map_plan_inverse"]
+_SIGNATURES["st_linear_supported"] = ([_INT, _INT, _INT], _INT)
+_SIGNATURES["st_linear_fwd"] = ([_INT, _PTR, _PTR, _PTR, _PTR, _I64, _INT, _INT, _PTR], _INT)
+_SIGNATURES["st_linear_dgrad"] = ([_INT, _PTR, _PTR, _PTR, _I64, _INT, _INT, _PTR], _INT)
+_SIGNATURES["st_linear_workspace_bytes"] = ([_I64, _INT, _INT], _I64)
+_SIGNATURES["st_linear_wgrad"] = ([_INT, _PTR, _PTR, _PTR, _PTR, _I64, _INT, _INT, _PTR, _I64, _PTR], _INT)
 _SIGNATURES["st_map_plan"] = ([_PTR, _I64, _INT, _INT, _PTR, _PTR, _PTR, _PTR, _I64, _PTR], _INT)
 _SIGNATURES["st_map_row_order_workspace_bytes"] = ([_I64, _INT], _I64)
 _SIGNATURES["st_map_row_order"] = ([_PTR, _I64, _INT, _PTR, _PTR, _I64, _PTR], _INT)

@@ -166,4 +166,4 @@ class SparseUNet(nn.Module):
             else:
                 x = skip_concat(up(x), skip)
             x = block(x)
-        return x.replace(self.head(x.F.float()))
+        return x.replace(self.head.float_rows(x.F))

@@ -235,3 +235,23 @@ def test_filtered_map_is_the_probed_map(cuda_device, ks, n):
                 _lib.check(L.st_map_build_symmetric_ws(p(c), n, code, off, K, shape, p(keys), p(vals), cap, p(out), None,
                                                        p(w) if w is not None else None, need if w is not None else 0, s), "map")
             assert torch.equal(a, b)
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16, torch.float32], ids=["bf16", "fp16", "fp32"])
+@pytest.mark.parametrize("n,C,O,bias", [(1, 16, 4, True), (63, 32, 20, True), (65, 64, 64, False), (5000, 32, 20, True),
+                                        (70001, 16, 64, True), (300000, 64, 12, False)])
+def test_row_linear(cuda_device, dtype, n, C, O, bias):
+    from sparsetriton_b200.nn.modules import SparseLinear
+    torch.manual_seed(n)
+    lin = SparseLinear(C, O, bias=bias).to(cuda_device)
+    x = torch.randn(n, C, device=cuda_device).to(dtype).requires_grad_(True)
+    y = lin.float_rows(x)
+    assert y.dtype == torch.float32
+    dy = torch.randn(n, O, device=cuda_device)
+    got = torch.autograd.grad(y, [x] + list(lin.parameters()), dy)
+    xd, w = x.detach().double(), lin.weight.detach().double()
+    want = [dy.double() @ w, dy.double().t() @ xd] + ([dy.double().sum(0)] if bias else [])
+    assert _rel(y, xd @ w.t() + (lin.bias.detach().double() if bias else 0)) < 1e-6
+    assert got[0].dtype == dtype and _rel(got[0], want[0]) < (1e-6 if dtype == torch.float32 else 3e-3)
+    for a, b in zip(got[1:], want[1:]):
+        assert _rel(a, b) < 1e-5
