@@ -359,11 +359,8 @@ def stage_rooflines(per_stage, n_in, n_out, pairs, pk, dtype, steps_fwd=0, steps
 # DRAM bytes (dram__bytes_read.sum + dram__bytes_write.sum) of one launch of the dominant kernels, from the ncu
 # captures summarised under profiles/ (default workload: 4 x 300 k voxels, bf16, stored-map algorithm).
 NCU_TRAFFIC_C3 = {
-    "conv_fwd": (466.4e6 + 187.8e6, "profiles/planned_gather_kernel_c3.md"),
-    "conv_dgrad": (820.9e6 + 143.0e6, "profiles/planned_gather_kernel_c3.md"),
-    # the stage's two kernels: the product and the sum of the partials (the copy of dY into tile order, 216.9 + 169.8 MB,
-    # runs on a second stream beside the feature gradient: stage conv_wgrad_presort)
-    "conv_wgrad": ((976.2e6 + 46.5e6) + (65.5e6 + 0.2e6), "profiles/planned_wgrad_kernel_c3.md"),
+    "conv_fwd": (391.2e6 + 154.0e6, "profiles/planned_products_bf16.md"),
+    "conv_wgrad": (640.2e6 + 4.1e6, "profiles/planned_products_bf16.md"),      # the product; its partial sums stay in L2
 }
 
 
