@@ -1548,9 +1548,13 @@ static bool plan_wgrad_planned(WgradPlan* plan, int dtype, int64_t n_rows, int K
   p.b_slots = std::min((budget - p.a_slots * p.a_slot_bytes) / p.b_slot_bytes, tc::kWgradBSlots3);
   // what lies behind the last tile slot must be shared memory too
   if (p.b_slots < 2 || (!swap && p.b_slots * p.b_slot_bytes < m_full - m_bytes)) return false;
-  // One CTA per SM (each writes its accumulators); with many combinations the shares would be too coarse: two.
+  // One CTA per SM (each writes its accumulators).  From an eighth of the SMs on in combinations the shares are too coarse: two,
+  // the second of an SM when its first is done, if there are tiles enough to pay for twice the partial sums.  (28 combinations, 747 and
+  // 918 tiles of 256 -> 256: 340 -> 319, 337 -> 304 us, but 123 tiles 88 -> 105; 14, 2450 tiles of 256 -> 128: 304 -> 325; four,
+  // 6370 tiles of 64 -> 128: 242 -> 262.)  From a third on, two in any case.
   const int combos = p.n_kgroups * p.n_coblk * p.n_ciblk;
-  int64_t ctas = combos * 3 <= sm_count() ? sm_count() : std::max(2 * sm_count(), combos);
+  const bool one = combos * 8 <= sm_count() || (combos * 3 <= sm_count() && p.n_tiles < 3 * sm_count());
+  int64_t ctas = one ? sm_count() : std::max(2 * sm_count(), combos);
   ctas = std::max<int64_t>(std::min<int64_t>(ctas, p.n_tiles * combos), combos);
   plan->n_chunks = (int)ctas;
   plan->smem = (size_t)p.a_slots * p.a_slot_bytes + (size_t)p.b_slots * p.b_slot_bytes + sizeof(tc::WgradControl3) + 1024;
